@@ -1,0 +1,76 @@
+"""Kernels and dispatch at the sizes where their tilings end: image tiles, line padding, layout
+copies, footprint columns and splat lattices, against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# float32 sums of a few hundred terms in another order than the oracle's, the parity bound of the
+# projectors
+PARITY = 1e-5
+
+
+def _apply(torch, proj, data, adjoint):
+    d = torch.from_numpy(np.ascontiguousarray(data, np.float32).ravel()).cuda()
+    out = torch.full((proj.domain_size if adjoint else proj.range_size,), float("nan"),
+                     device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    (proj.apply_adjoint_ptr if adjoint else proj.apply_ptr)(d.data_ptr(), out.data_ptr(), s)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _problem(oracle, vol, views, det, arc=360, seed=3):
+    n = max(vol)
+    poses, det = oracle.circle_trajectory(vol, views, arc, 5.0 * n, 1.5 * n, det)
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0, 1, int(np.prod(vol))).astype(np.float32)
+    y = rng.uniform(0, 1, int(np.prod(det))).astype(np.float32)
+    return poses, det, x, y
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kind,params", [
+    ("blob", (2.0, 10.83, 2)), ("blob", (0.55, 10.83, 2)), ("blob", (3.7, 8.0, 1)),
+    ("blob", (9.0, 10.83, 2)), ("blob", (1.3, 2.0, 0)), ("bspline", (0,)), ("bspline", (5,)),
+    ("phase_blob", (3.1, 10.83, 2)), ("phase_bspline", (3,))])
+@pytest.mark.parametrize("vol,views,det", [((13, 21, 9), 7, [17, 12]), ((50, 6, 49), 5, [70, 31]),
+                                           ((200, 7), 6, [90])])
+def test_voxel_footprints(cuda, oracle, vol, views, det, kind, params, mode):
+    """Footprints of one pixel to more than six columns, lattices that overlap (shared atomics),
+    patches that do not fit, tables that do not end in 0, voxels projected off the detector. The
+    default adjoint visits exactly the pixels of the exact one: its weights differ by a few ulp
+    (an edge pixel more or less would show as 1e-4)."""
+    import elsa_b200
+    codes = {"blob": 2, "bspline": 3, "phase_blob": 4, "phase_bspline": 5}
+    poses, det, x, y = _problem(oracle, vol, views, det)
+    x[::3] = 0.0
+    proj = elsa_b200.Projector(codes[kind], vol, det, poses, tuple(map(float, params)) + (mode,))
+    if kind.endswith("blob"):
+        lut, support, wk = oracle.voxel_lut(kind, len(vol), *params)
+    else:
+        lut, support, wk = oracle.voxel_lut(kind, len(vol), order=params[0])
+    args = (vol, det, poses, lut, support, wk, mode)
+    ref = oracle.voxel_project(False, x, *args)
+    assert rel_l2(_apply(cuda, proj, x, False), ref) <= PARITY
+    fast = _apply(cuda, proj, y, True)
+    proj.set_knob(elsa_b200.KNOB_EXACT_WEIGHTS, 1)
+    exact = _apply(cuda, proj, y, True)
+    assert np.array_equal(exact, np.asarray(oracle.voxel_project(True, y, *args), np.float32))
+    # phase-contrast sums cancel: weights of both signs, relative to their magnitude
+    assert rel_l2(fast, exact) <= (PARITY if kind.startswith("phase") else 2e-6)
+
+
+def test_voxel_adjoint_same_footprints_at_size(cuda, oracle):
+    """10^8 footprints: one ulp in a centre or a scaling would move the edges of about a thousand
+    of them and the sums by 1e-5 and more."""
+    import elsa_b200
+    vol = (128, 128, 64)
+    poses, det = oracle.circle_trajectory(vol, 96, 360, 1280.0, 320.0, [192, 96])
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_BLOB, vol, det, poses)
+    y = np.random.default_rng(1).uniform(0, 1, int(np.prod(det))).astype(np.float32)
+    fast = _apply(cuda, proj, y, True)
+    proj.set_knob(elsa_b200.KNOB_EXACT_WEIGHTS, 1)
+    assert rel_l2(fast, _apply(cuda, proj, y, True)) <= 5e-7
