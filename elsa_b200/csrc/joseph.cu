@@ -1005,251 +1005,102 @@ namespace elsa_b200
         // neighbouring brick owns it); with ELSA_AXIS_HALO 2 the brick instead carries a two-voxel
         // halo into which tap indices are clamped, and the halo is not written out.
         // ---------------------------------------------------------------------------------------
-#ifndef ELSA_AXIS_HALO
-// halo of the axis bricks: 0, taps outside the brick predicated off (256^3: 35.9 ms); 2, taps
-// clamped into a two-voxel halo (38.9 ms with 8-deep bricks, whose halo costs occupancy)
-#define ELSA_AXIS_HALO 0
-#endif
-        constexpr int kAxisHalo = ELSA_AXIS_HALO;
-        static_assert(kAxisHalo == 0 || kAxisHalo == 2, "halo of 0 or 2 voxels");
-
         // Shared-memory brick of TD planes (along G) of TV rows x TW columns. Columns run along
         // the non-driving axis over which the rays of a detector row spread (the warp's lanes
         // spread along it, so stride 1 there keeps their taps in different banks), rows along the
-        // other one; both carry the halo.
-#ifndef ELSA_ADJ_PACKED
-#define ELSA_ADJ_PACKED 1 // the (a, b) pairs on the packed two-wide FP32 instructions (256^3:
-                          // 32.92 -> 32.17 ms, the same adjoint bit for bit)
-#endif
-#ifndef ELSA_AXIS_PLANE_ODD
-#define ELSA_AXIS_PLANE_ODD 0 // 1: pad the plane stride to 1 modulo 32 (256^3: 35.8 ms, 0: 33.5 ms)
-#endif
-#ifndef ELSA_AXIS_ROWPAD
-#define ELSA_AXIS_ROWPAD (ELSA_AXIS_HALO == 0 ? 1 : 0) // extra words per row (bank spread)
-#endif
+        // other one. A halo column on either side takes the taps of samples that straddle the
+        // brick's edge (they belong to the neighbouring brick and are not written out), so that
+        // the four taps of a sample need two predicates, one per row, instead of four and a mask of
+        // them carried along. 48 instructions per step of 32 rays instead of 62: 256^3 / 360 views /
+        // 384^2 32.2 -> 28.2 ms, now bound by the shared-memory pipe (78 %; half of its wavefronts
+        // are bank conflicts between the rows of a class). Rows of 35 words: 29.1 ms; 7 or 10 rows:
+        // 28.6 / 30.2; 2 or 4 rays fetched per lane: 28.4 / 28.5; unrolled 1 or 4: 31.7 / 28.3.
         template <int TD, int TW, int TV>
         struct AxisBrick {
-            // words per row (stride 1 axis)
-            static constexpr int kRow = TW + 2 * kAxisHalo + ELSA_AXIS_ROWPAD;
-            static constexpr int kRows = TV + 2 * kAxisHalo; // rows per plane
-            static constexpr int kPlaneMin = kRow * kRows;
-            // plane stride unpadded (smaller bricks, more of them resident per SM), or congruent
-            // to 1 modulo 32 with ELSA_AXIS_PLANE_ODD 1 (lanes one plane apart in other banks)
-            static constexpr int kPlane =
-                ELSA_AXIS_PLANE_ODD ? kPlaneMin + ((33 - kPlaneMin % 32) % 32) : kPlaneMin;
+            static constexpr int kRow = TW + 2; // words per row
+            static constexpr int kPlane = kRow * TV;
             static constexpr int kWords = kPlane * TD;
         };
 
-        // Axis roles of an axis brick: non-driving axes a < b of G; UB: the columns run along b
-        // (else along a). Edges and word strides along a and b.
+        // Word of the voxel (a, b) of an axis brick's plane: a < b the non-driving axes of G; UB:
+        // the columns run along b (else along a).
         template <int TD, bool UB, int TW, int TV>
         struct AxisRolesAB {
             using L = AxisBrick<TD, TW, TV>;
-            static constexpr int EA = UB ? TV : TW, EB = UB ? TW : TV;
             static constexpr int SA = UB ? L::kRow : 1, SB = UB ? 1 : L::kRow;
-            static constexpr int kOrigin = kAxisHalo * (SA + SB); // word of (a, b) = (0, 0)
+            static constexpr int kOrigin = 1; // word of (a, b) = (0, 0)
         };
 
-        // Word of the bilinear footprint of position (pa, pb) on `plane` (the brick word of
-        // a = b = 0 on that plane) and the reference's weights (JosephsMethod.cpp:37-52); tap
-        // indices outside the brick are clamped into the halo.
-        template <int EA, int EB, int SA, int SB>
-        __device__ __forceinline__ float* axisTap(float* plane, float pa, float pb, int orgA,
-                                                  int orgB, float& wa, float& cwa, float& wb,
-                                                  float& cwb)
-        {
-            const float fa = floorf(__fsub_rn(pa, 0.5f));
-            const float fb = floorf(__fsub_rn(pb, 0.5f));
-            cwa = __fsub_rn(__fsub_rn(pa, fa), 0.5f);
-            cwb = __fsub_rn(__fsub_rn(pb, fb), 0.5f);
-            wa = __fsub_rn(1.0f, cwa);
-            wb = __fsub_rn(1.0f, cwb);
-            const int la = min(max(static_cast<int>(fa) - orgA, -kAxisHalo), EA);
-            const int lb = min(max(static_cast<int>(fb) - orgB, -kAxisHalo), EB);
-            return plane + la * SA + lb * SB;
-        }
-
-        // Without a halo: the word offset of the footprint on its plane and a mask of the taps
-        // inside the brick (bit t: tap (a + (t & 1), b + (t >> 1))).
-        template <int EA, int EB, int SA, int SB>
-        __device__ __forceinline__ int axisTapMasked(float pa, float pb, int orgA, int orgB,
-                                                     float& wa, float& cwa, float& wb, float& cwb,
-                                                     unsigned& mask)
-        {
-            // (floorSmall here, instead of floorf and a conversion: 256^3 33.3 ms against 32.9)
-            const float fa = floorf(__fsub_rn(pa, 0.5f));
-            const float fb = floorf(__fsub_rn(pb, 0.5f));
-            const int ia = static_cast<int>(fa), ib = static_cast<int>(fb);
-            cwa = __fsub_rn(__fsub_rn(pa, fa), 0.5f);
-            cwb = __fsub_rn(__fsub_rn(pb, fb), 0.5f);
-            wa = __fsub_rn(1.0f, cwa);
-            wb = __fsub_rn(1.0f, cwb);
-            const int la = ia - orgA, lb = ib - orgB;
-            const bool a0 = static_cast<unsigned>(la) < static_cast<unsigned>(EA);
-            const bool a1 = static_cast<unsigned>(la + 1) < static_cast<unsigned>(EA);
-            const bool b0 = static_cast<unsigned>(lb) < static_cast<unsigned>(EB);
-            const bool b1 = static_cast<unsigned>(lb + 1) < static_cast<unsigned>(EB);
-            mask = (a0 && b0 ? 1u : 0u) | (a1 && b0 ? 2u : 0u) | (a0 && b1 ? 4u : 0u) |
-                   (a1 && b1 ? 8u : 0u);
-            return la * SA + lb * SB;
-        }
-
         // Samples jLo..jHi of ray R (position cp at sample jLo, on brick plane t0) into the brick.
-        // Software-pipelined: the footprint of sample j+1 (always on another plane) is read before
-        // the sums of sample j are written back.
+        // (column, row) pairs run on the packed two-wide FP32 instructions with the reference's
+        // roundings (JosephsMethod.cpp:37-52; the weight (p - floor) - 0.5 as (p - 0.5) - floor,
+        // the same number for p >= 1). Software-pipelined: the footprint of sample j+1 (always on
+        // another plane) is read before the sums of sample j are written back.
         template <int TD, bool UB, int TW, int TV>
         __device__ __forceinline__ void axisSplat(float* acc, const JosephRay& R, float yl,
                                                   float2 cp, int jLo, int jHi, int t0, int orgA,
                                                   int orgB)
         {
             using L = AxisBrick<TD, TW, TV>;
-            using AR = AxisRolesAB<TD, UB, TW, TV>;
-            constexpr int SA = AR::SA, SB = AR::SB;
-#if ELSA_ADJ_PACKED
-            if constexpr (kAxisHalo == 0) {
-                // (a, b) pairs on the packed two-wide FP32 instructions: the same roundings
-                const int dPlane = ((R.meta & 4) ? -1 : 1) * L::kPlane;
-                const float2 h = make_float2(0.5f, 0.5f), one = make_float2(1.0f, 1.0f);
-                const float2 s2 = make_float2(R.sa, R.sb), yy = make_float2(yl, yl);
-                int plane = t0 * L::kPlane;
-                float2 p2 = cp;
-                auto tap = [&](int pl, float2& w, float2& cw, unsigned& mk) {
-                    int ia, ib;
-                    const float2 fl = floorSmall2(sub2(p2, h), ia, ib);
-                    cw = sub2(sub2(p2, fl), h);
-                    w = sub2(one, cw);
-                    const int la = ia - orgA, lb = ib - orgB;
-                    const bool a0 = static_cast<unsigned>(la) < static_cast<unsigned>(AR::EA);
-                    const bool a1 = static_cast<unsigned>(la + 1) < static_cast<unsigned>(AR::EA);
-                    const bool b0 = static_cast<unsigned>(lb) < static_cast<unsigned>(AR::EB);
-                    const bool b1 = static_cast<unsigned>(lb + 1) < static_cast<unsigned>(AR::EB);
-                    mk = (a0 && b0 ? 1u : 0u) | (a1 && b0 ? 2u : 0u) | (a0 && b1 ? 4u : 0u) |
-                         (a1 && b1 ? 8u : 0u);
-                    return pl + la * SA + lb * SB;
-                };
-                float2 w, cw;
-                unsigned mk;
-                int o = tap(plane, w, cw, mk);
-                float2 v01 = make_float2((mk & 1u) ? acc[o] : 0.0f, (mk & 2u) ? acc[o + SA] : 0.0f);
-                float2 v23 = make_float2((mk & 4u) ? acc[o + SB] : 0.0f,
-                                         (mk & 8u) ? acc[o + SA + SB] : 0.0f);
-                float2 yac = mul2(yy, make_float2(w.x, cw.x)); // (ya, yc)
-                float wb = w.y, cwb = cw.y;
-#pragma unroll kSplatUnroll
-                for (int j = jLo; j < jHi; ++j) {
-                    plane += dPlane;
-                    p2 = add2(p2, s2);
-                    float2 w2, cw2;
-                    unsigned mk2;
-                    const int o2 = tap(plane, w2, cw2, mk2);
-                    const float2 n01 = make_float2((mk2 & 1u) ? acc[o2] : 0.0f,
-                                                   (mk2 & 2u) ? acc[o2 + SA] : 0.0f);
-                    const float2 n23 = make_float2((mk2 & 4u) ? acc[o2 + SB] : 0.0f,
-                                                   (mk2 & 8u) ? acc[o2 + SA + SB] : 0.0f);
-                    const float2 r01 = fma2(yac, make_float2(wb, wb), v01);
-                    const float2 r23 = fma2(yac, make_float2(cwb, cwb), v23);
-                    if (mk & 1u)
-                        acc[o] = r01.x;
-                    if (mk & 2u)
-                        acc[o + SA] = r01.y;
-                    if (mk & 4u)
-                        acc[o + SB] = r23.x;
-                    if (mk & 8u)
-                        acc[o + SA + SB] = r23.y;
-                    o = o2, mk = mk2;
-                    v01 = n01, v23 = n23;
-                    yac = mul2(yy, make_float2(w2.x, cw2.x));
-                    wb = w2.y, cwb = cw2.y;
-                }
-                const float2 r01 = fma2(yac, make_float2(wb, wb), v01);
-                const float2 r23 = fma2(yac, make_float2(cwb, cwb), v23);
-                if (mk & 1u)
-                    acc[o] = r01.x;
-                if (mk & 2u)
-                    acc[o + SA] = r01.y;
-                if (mk & 4u)
-                    acc[o + SB] = r23.x;
-                if (mk & 8u)
-                    acc[o + SA + SB] = r23.y;
-                return;
-            }
-#endif
-            if constexpr (kAxisHalo == 0) {
-                const int dPlane = ((R.meta & 4) ? -1 : 1) * L::kPlane;
-                int plane = t0 * L::kPlane;
-                float pa = cp.x, pb = cp.y;
-                float wa, cwa, wb, cwb;
-                unsigned mk;
-                int o = plane + axisTapMasked<AR::EA, AR::EB, SA, SB>(pa, pb, orgA, orgB, wa, cwa,
-                                                                       wb, cwb, mk);
-                float v0 = (mk & 1u) ? acc[o] : 0.0f, v1 = (mk & 2u) ? acc[o + SA] : 0.0f;
-                float v2 = (mk & 4u) ? acc[o + SB] : 0.0f, v3 = (mk & 8u) ? acc[o + SA + SB] : 0.0f;
-                float ya = yl * wa, yc = yl * cwa;
-#pragma unroll kSplatUnroll
-                for (int j = jLo; j < jHi; ++j) {
-                    plane += dPlane;
-                    pa = __fadd_rn(pa, R.sa);
-                    pb = __fadd_rn(pb, R.sb);
-                    float wa2, cwa2, wb2, cwb2;
-                    unsigned mk2;
-                    const int o2 = plane + axisTapMasked<AR::EA, AR::EB, SA, SB>(
-                                               pa, pb, orgA, orgB, wa2, cwa2, wb2, cwb2, mk2);
-                    const float n0 = (mk2 & 1u) ? acc[o2] : 0.0f;
-                    const float n1 = (mk2 & 2u) ? acc[o2 + SA] : 0.0f;
-                    const float n2 = (mk2 & 4u) ? acc[o2 + SB] : 0.0f;
-                    const float n3 = (mk2 & 8u) ? acc[o2 + SA + SB] : 0.0f;
-                    if (mk & 1u)
-                        acc[o] = v0 + ya * wb;
-                    if (mk & 2u)
-                        acc[o + SA] = v1 + yc * wb;
-                    if (mk & 4u)
-                        acc[o + SB] = v2 + ya * cwb;
-                    if (mk & 8u)
-                        acc[o + SA + SB] = v3 + yc * cwb;
-                    o = o2, mk = mk2;
-                    v0 = n0, v1 = n1, v2 = n2, v3 = n3;
-                    ya = yl * wa2, yc = yl * cwa2;
-                    wb = wb2, cwb = cwb2;
-                }
-                if (mk & 1u)
-                    acc[o] = v0 + ya * wb;
-                if (mk & 2u)
-                    acc[o + SA] = v1 + yc * wb;
-                if (mk & 4u)
-                    acc[o + SB] = v2 + ya * cwb;
-                if (mk & 8u)
-                    acc[o + SA + SB] = v3 + yc * cwb;
-                return;
-            }
+            constexpr int kRow = L::kRow;
+            const float2 half = splat2(0.5f), one = splat2(1.0f), magic = splat2(12582912.0f);
+            const float2 s2 = UB ? make_float2(R.sb, R.sa) : make_float2(R.sa, R.sb);
+            float2 p2 = UB ? make_float2(cp.y, cp.x) : cp;
+            // floor(p - 0.5) + 1 - origin of the columns (the halo column is 0), floor(p - 0.5) -
+            // origin of the rows, from the bit patterns of the floors (floorSmall2)
+            const unsigned biasC = 0x4B400000u + static_cast<unsigned>(UB ? orgB : orgA) - 1u;
+            const unsigned biasR = 0x4B400000u + static_cast<unsigned>(UB ? orgA : orgB);
             const int dPlane = ((R.meta & 4) ? -1 : 1) * L::kPlane;
-            float* plane = acc + AR::kOrigin + t0 * L::kPlane;
-            float pa = cp.x, pb = cp.y;
-            float wa, cwa, wb, cwb;
-            float* q = axisTap<AR::EA, AR::EB, SA, SB>(plane, pa, pb, orgA, orgB, wa, cwa, wb, cwb);
-            float v0 = q[0], v1 = q[SA], v2 = q[SB], v3 = q[SA + SB];
-            float ya = yl * wa, yc = yl * cwa;
+            int plane = t0 * L::kPlane;
+            struct Tap {
+                int o;      // word of the footprint's first tap
+                bool r0, r1; // its rows lie in the brick
+                float2 w, cw;
+            };
+            auto tap = [&]() {
+                Tap t;
+                const float2 h = sub2(p2, half);
+                const float2 f = add2Down(h, magic);
+                t.cw = sub2(h, sub2(f, magic));
+                t.w = sub2(one, t.cw);
+                const unsigned c = __float_as_uint(f.x) - biasC, r = __float_as_uint(f.y) - biasR;
+                const bool in = c < static_cast<unsigned>(TW + 1);
+                t.r0 = in && r < static_cast<unsigned>(TV);
+                t.r1 = in && r + 1u < static_cast<unsigned>(TV);
+                t.o = plane + static_cast<int>(r * kRow + c);
+                return t;
+            };
+            Tap t = tap();
+            float2 v0 = splat2(0.0f), v1 = splat2(0.0f);
+            if (t.r0)
+                v0 = make_float2(acc[t.o], acc[t.o + 1]);
+            if (t.r1)
+                v1 = make_float2(acc[t.o + kRow], acc[t.o + kRow + 1]);
+            auto store = [&]() {
+                const float ya = yl * t.w.x, yc = yl * t.cw.x;
+                if (t.r0) {
+                    acc[t.o] = __fmaf_rn(ya, t.w.y, v0.x);
+                    acc[t.o + 1] = __fmaf_rn(yc, t.w.y, v0.y);
+                }
+                if (t.r1) {
+                    acc[t.o + kRow] = __fmaf_rn(ya, t.cw.y, v1.x);
+                    acc[t.o + kRow + 1] = __fmaf_rn(yc, t.cw.y, v1.y);
+                }
+            };
 #pragma unroll kSplatUnroll
             for (int j = jLo; j < jHi; ++j) {
                 plane += dPlane;
-                pa = __fadd_rn(pa, R.sa);
-                pb = __fadd_rn(pb, R.sb);
-                float wa2, cwa2, wb2, cwb2;
-                float* q2 = axisTap<AR::EA, AR::EB, SA, SB>(plane, pa, pb, orgA, orgB, wa2, cwa2,
-                                                           wb2, cwb2);
-                const float n0 = q2[0], n1 = q2[SA], n2 = q2[SB], n3 = q2[SA + SB];
-                q[0] = v0 + ya * wb;
-                q[SA] = v1 + yc * wb;
-                q[SB] = v2 + ya * cwb;
-                q[SA + SB] = v3 + yc * cwb;
-                q = q2;
-                v0 = n0, v1 = n1, v2 = n2, v3 = n3;
-                ya = yl * wa2, yc = yl * cwa2;
-                wb = wb2, cwb = cwb2;
+                p2 = add2(p2, s2);
+                const Tap n = tap();
+                float2 n0 = splat2(0.0f), n1 = splat2(0.0f);
+                if (n.r0)
+                    n0 = make_float2(acc[n.o], acc[n.o + 1]);
+                if (n.r1)
+                    n1 = make_float2(acc[n.o + kRow], acc[n.o + kRow + 1]);
+                store();
+                t = n, v0 = n0, v1 = n1;
             }
-            q[0] = v0 + ya * wb;
-            q[SA] = v1 + yc * wb;
-            q[SB] = v2 + ya * cwb;
-            q[SA + SB] = v3 + yc * cwb;
+            store();
         }
 
         // One view for an axis brick of grid G: m x m ray classes separated by __syncwarp; lane i
