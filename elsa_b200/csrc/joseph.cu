@@ -16,21 +16,22 @@
 // ray's first sample in each slab of kCheckpointDepth planes, computed once per geometry) and
 // accumulates from there.
 //
-// Forward: one thread per ray, samples gathered through the read-only cache (the volume is
-// L2-resident: 67 MB at 256^3 against a 126 MB L2).
+// Forward: joseph_tma.cu in 3D; in 2D a warp takes 32 neighbouring rays through a checkpoint slab,
+// reading zero-padded copies of the image's rows and columns.
 //
-// Adjoint (default): atomic-free and deterministic. Each CTA owns one brick of the volume in shared memory
-// for all views. For every view it visits the rays of the brick's detector window one
-// conflict-free class at a time: rays whose pixel indices are congruent modulo m stay more than
-// two voxels apart on every plane (m is validated per geometry at construction), so their
-// bilinear taps never overlap and the threads update shared memory without atomics. Each thread
-// walks one ray through the brick; classes are separated by barriers. Every voxel receives its
-// contributions in a fixed order, with exactly the positions and weights of the forward kernel.
+// Adjoint (default): atomic-free and deterministic. Each warp owns one brick (2D: tile) of the
+// volume in shared memory for a chunk of the views. For every view it visits the rays of the
+// brick's detector window so that lanes never meet: rays whose pixel indices are congruent modulo
+// m stay more than two voxels apart on every plane (m is validated per geometry at construction),
+// so their bilinear taps never overlap and shared memory is updated without atomics. In 3D the
+// lanes take one such class at a time; in 2D 32 neighbouring rays, those of different classes on
+// different planes. Every voxel receives its contributions in a fixed order, with the positions
+// and weights of the forward kernel.
 // The launch knob kKnobAdjointScatter = 1 selects a thread-per-ray scatter instead (the forward's
-// sample loop with atomic adds to the four taps): faster in 2D, slower in 3D, where four global
-// atomics per sample exceed what the L2 sustains. A shared-memory variant (several warps per
-// brick adding with shared atomics, no ray classes) measured 65.5 ms against 54.8 ms at
-// 256^3 / 360 views and was dropped.
+// sample loop with atomic adds to the four taps), slower in 2D (512^2 / 720 views: 1.74 ms against
+// 0.51) and 3D, where four global atomics per sample exceed what the L2 sustains. A shared-memory
+// variant (several warps per brick adding with shared atomics, no ray classes) measured 65.5 ms
+// against 54.8 ms at 256^3 / 360 views and was dropped.
 #include "joseph_tma.cuh"
 #include "projector.hpp"
 #include "raysetup.cuh"
@@ -103,61 +104,6 @@ namespace elsa_b200
         __device__ __forceinline__ int floorDiv(int a, int b)
         {
             return a >= 0 ? a / b : -((-a + b - 1) / b);
-        }
-
-        template <int DIM>
-        __global__ void __launch_bounds__(kMaxForwardThreads)
-            josephForwardKernel(const JosephRay* __restrict__ rays, int64_t nrays,
-                                const float* __restrict__ x, VolumeShape vol,
-                                float* __restrict__ y)
-        {
-            const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (r >= nrays)
-                return;
-            const JosephRay R = rays[r];
-            if (R.n == 0) {
-                y[r] = 0.0f;
-                return;
-            }
-            const int g = R.meta & 3;
-            const int dir = (R.meta & 4) ? -1 : 1;
-            int a, b;
-            nonDrivingAxes(g, a, b);
-            const int64_t plane = static_cast<int64_t>(vol.n[0]) * vol.n[1];
-            const int64_t sg = g == 0 ? 1 : (g == 1 ? vol.n[0] : plane);
-            const int64_t sa = a == 0 ? 1 : (a == 1 ? vol.n[0] : plane);
-            const int ng = g == 0 ? vol.n[0] : (g == 1 ? vol.n[1] : vol.n[2]);
-            const int na = a == 0 ? vol.n[0] : (a == 1 ? vol.n[1] : vol.n[2]);
-            const int64_t sb = DIM == 3 ? (b == 1 ? vol.n[0] : plane) : 0;
-            const int nb = DIM == 3 ? (b == 1 ? vol.n[1] : vol.n[2]) : 1;
-            float acc = 0.0f;
-            float pa = R.pa, pb = R.pb;
-            int k = R.k0;
-            for (int j = 0; j < R.n; ++j, k += dir, pa = __fadd_rn(pa, R.sa),
-                     pb = __fadd_rn(pb, R.sb)) {
-                if (static_cast<unsigned>(k) >= static_cast<unsigned>(ng))
-                    continue;
-                Weights w;
-                tapWeights(pa, pb, w);
-                const float* base = x + k * sg;
-                const bool a0 = static_cast<unsigned>(w.ia) < static_cast<unsigned>(na);
-                const bool a1 = static_cast<unsigned>(w.ia + 1) < static_cast<unsigned>(na);
-                if (DIM == 2) {
-                    const float v0 = a0 ? __ldg(base + w.ia * sa) : 0.0f;
-                    const float v1 = a1 ? __ldg(base + (w.ia + 1) * sa) : 0.0f;
-                    acc += w.wa * v0 + w.cwa * v1;
-                } else {
-                    const bool b0 = static_cast<unsigned>(w.ib) < static_cast<unsigned>(nb);
-                    const bool b1 = static_cast<unsigned>(w.ib + 1) < static_cast<unsigned>(nb);
-                    const float* p0 = base + w.ia * sa + w.ib * sb;
-                    const float v00 = (a0 && b0) ? __ldg(p0) : 0.0f;
-                    const float v10 = (a1 && b0) ? __ldg(p0 + sa) : 0.0f;
-                    const float v01 = (a0 && b1) ? __ldg(p0 + sb) : 0.0f;
-                    const float v11 = (a1 && b1) ? __ldg(p0 + sa + sb) : 0.0f;
-                    acc += w.wb * (w.wa * v00 + w.cwa * v10) + w.cwb * (w.wa * v01 + w.cwa * v11);
-                }
-            }
-            y[r] = R.len * acc;
         }
 
         // Adjoint by atomic scatter: the forward's sample loop, one thread per ray, adding
@@ -632,262 +578,248 @@ namespace elsa_b200
             return jLo <= jHi;
         }
 
-        // Strides of the shared-memory brick (x fastest; the plane stride is padded by one word
-        // so that neighbouring rays stepping along z or x hit different banks).
-        template <int DIM, int BX, int BY>
-        struct BrickLayout {
-            static constexpr int kRow = DIM == 3 ? BX : BX + 1;
-            static constexpr int kPlane = DIM == 3 ? BX * BY + 1 : kRow * BY;
-        };
+        // ---- 2D on padded copies and square tiles ------------------------------------------------
+        // Forward. A sample of a ray along axis G reads two neighbouring pixels of image line k
+        // (a row for G = y, a column for G = x). The image is copied twice per call, as rows and
+        // as columns, each line between kLinePad zeros, so that the 32 neighbouring rays of a
+        // warp read consecutive words whatever their axis and taps outside the image need no
+        // test. A warp takes 32 rays through one checkpoint slab of planes, starting from the
+        // exact accumulated positions of the checkpoints; the slabs' sums are added in slab
+        // order. Bound by issue and L2 latency: one thread per ray reading the image itself took
+        // 0.87 ms at 512^2 / 720 views / 730 pixels (half of the views read one word per sector),
+        // this takes 0.23 ms.
+        constexpr int kLinePad = 8;
+        __host__ __device__ inline int linePitch(int n) { return (n + 2 * kLinePad + 3) / 4 * 4; }
 
-        // Axis roles for driving axis G: stride/extent of G and of the non-driving axes a < b.
-        template <int DIM, int G, int BX, int BY, int BZ>
-        struct AxisRoles {
-            using L = BrickLayout<DIM, BX, BY>;
-            static constexpr int strG = G == 0 ? 1 : (G == 1 ? L::kRow : L::kPlane);
-            static constexpr int extG = G == 0 ? BX : (G == 1 ? BY : BZ);
-            static constexpr int strA = G == 0 ? L::kRow : 1;
-            static constexpr int extA = G == 0 ? BY : BX;
-            static constexpr int strB = DIM == 2 ? 0 : (G == 2 ? L::kRow : L::kPlane);
-            static constexpr int extB = DIM == 2 ? 1 : (G == 2 ? BY : BZ);
-        };
-
-        // Add to the brick word at local lane-axis column L, row-axis row O (if inside).
-        template <int EXT_L, int EXT_O, int STR_L, int STR_O>
-        __device__ __forceinline__ void addTap(float* plane, int L, int O, float v)
+        // rows: ny lines of linePitch(nx); columns: nx lines of linePitch(ny). 32 x 8 threads per
+        // 32 x 32 block of the image.
+        __global__ void padLinesKernel(const float* __restrict__ x, int nx, int ny,
+                                       float* __restrict__ rows, float* __restrict__ columns)
         {
-            if (static_cast<unsigned>(L) < static_cast<unsigned>(EXT_L) &&
-                static_cast<unsigned>(O) < static_cast<unsigned>(EXT_O)) {
-                float* q = plane + L * STR_L + O * STR_O;
-                *q = *q + v;
+            __shared__ float t[32][33];
+            const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+            const int pitchX = linePitch(nx), pitchY = linePitch(ny);
+            for (int j = threadIdx.y; j < 32; j += 8) {
+                const int ix = x0 + threadIdx.x, iy = y0 + j;
+                const float v =
+                    ix < nx && iy < ny ? x[ix + static_cast<int64_t>(nx) * iy] : 0.0f;
+                t[j][threadIdx.x] = v;
+                if (ix < nx && iy < ny)
+                    rows[static_cast<int64_t>(iy) * pitchX + kLinePad + ix] = v;
+            }
+            __syncthreads();
+            for (int j = threadIdx.y; j < 32; j += 8) {
+                const int ix = x0 + j, iy = y0 + threadIdx.x;
+                if (ix < nx && iy < ny)
+                    columns[static_cast<int64_t>(ix) * pitchY + kLinePad + iy] = t[threadIdx.x][j];
             }
         }
 
-        // One warp splats 32 neighbouring rays (u = uSeg0 + lane) of detector row v through the
-        // brick, plane by plane in ray order. Lanes spread along the "lane axis" (a, or b when
-        // LB); taps landing in the same column are merged across neighbouring lanes, then the
-        // first and the second column of every lane's bilinear footprint are written in two
-        // separate phases, so no two lanes touch the same word at the same time. When the merge
-        // precondition fails (two neighbours on one column but different rows, or three on one
-        // column) the plane falls back to m phases of lanes m apart, which the class check proves
-        // disjoint.
-        template <int DIM, int G, bool LB, int BX, int BY, int BZ, int CPD>
-        __device__ __forceinline__ void splatRowSegment(
-            float* acc, const JosephRay* __restrict__ rays, const float2* __restrict__ cps,
-            int64_t nrays, const float* __restrict__ y, const DetectorShape& det, int p, int v,
-            int uSeg0, int u1, int m, int orgG, int orgA, int orgB)
+        // `count` samples from position p on, line `q` (its pixel 0) advancing by `lineStep`.
+        template <bool Clamp>
+        __device__ __forceinline__ float lineSamples(const float* q, int64_t lineStep, float p,
+                                                     float s, int count, int n)
         {
-            using AR = AxisRoles<DIM, G, BX, BY, BZ>;
-            constexpr int EXT_L = LB ? AR::extB : AR::extA;
-            constexpr int EXT_O = LB ? AR::extA : AR::extB;
-            constexpr int STR_L = LB ? AR::strB : AR::strA;
-            constexpr int STR_O = LB ? AR::strA : AR::strB;
-            const int lane = threadIdx.x & 31;
-            const int u = uSeg0 + lane;
-            const int kLo = orgG, kHi = orgG + AR::extG - 1;
-            const int64_t r =
-                u + static_cast<int64_t>(det.nu) * (v + static_cast<int64_t>(det.nv) * p);
+            float acc = 0.0f;
+#pragma unroll 8
+            for (int j = 0; j < count; ++j) {
+                int i;
+                const float h = __fsub_rn(p, 0.5f);
+                const float cw = __fsub_rn(h, floorSmall(h, i));
+                if (Clamp)
+                    i = min(max(i, -2), n);
+                acc = __fmaf_rn(__fsub_rn(1.0f, cw), __ldg(q + i), acc);
+                acc = __fmaf_rn(cw, __ldg(q + i + 1), acc);
+                p = __fadd_rn(p, s);
+                q += lineStep;
+            }
+            return acc;
+        }
+
+        // blockDim.x = 32 lanes (neighbouring rays of one view), blockDim.y = warps: `groups` groups
+        // of warps, one view each, the warps of a group dividing its slabs. A block's views follow
+        // one another, so its groups read nearly the same lines from L1.
+        __global__ void __launch_bounds__(kMaxForwardThreads)
+            josephForward2dKernel(const JosephRay* __restrict__ rays,
+                                  const float2* __restrict__ checkpoints, int64_t nrays,
+                                  VolumeShape vol, DetectorShape det, int depth, int nSlabs,
+                                  int groups, int segments, const float* __restrict__ rows,
+                                  const float* __restrict__ columns, float* __restrict__ y)
+        {
+            __shared__ float sums[kMaxForwardThreads];
+            const int lane = threadIdx.x;
+            const int perGroup = blockDim.y / groups;
+            const int group = threadIdx.y / perGroup, member = threadIdx.y - group * perGroup;
+            const int p = static_cast<int>(blockIdx.x / segments) * groups + group;
+            const int u = static_cast<int>(blockIdx.x % segments) * 32 + lane;
+            const bool valid = p < det.np && u < det.nu;
+            const int64_t r = u + static_cast<int64_t>(det.nu) * p;
+            JosephRay R{};
+            if (valid)
+                R = rays[r];
+            const int g = R.meta & 3;
+            const int dir = (R.meta & 4) ? -1 : 1;
+            const int n = g == 0 ? vol.n[1] : vol.n[0], ng = g == 0 ? vol.n[0] : vol.n[1];
+            const int pitch = linePitch(n);
+            const float* lines = (g == 0 ? columns : rows) + kLinePad;
+            float acc = 0.0f;
+            for (int slab = member; slab < nSlabs; slab += perGroup) {
+                int jLo, jHi;
+                if (R.n == 0 || !sampleRange(R, slab * depth, (slab + 1) * depth - 1, jLo, jHi))
+                    continue;
+                int k = R.k0 + jLo * dir, count = jHi - jLo + 1;
+                float pos = __ldg(checkpoints + (slab + 1) * nrays + r).x;
+                // samples past the image's last line (a ray may start on its far face)
+                for (; dir < 0 && k >= ng && count > 0; --k, --count)
+                    pos = __fadd_rn(pos, R.sa);
+                if (dir > 0)
+                    count = min(count, ng - k);
+                // positions are monotone along the ray; a sample's line words are within the
+                // padding unless the positions leave the image by several voxels
+                const float end = pos + R.sa * static_cast<float>(count);
+                const float far = static_cast<float>(n) + 4.0f;
+                const bool inside = pos > -4.0f && pos < far && end > -4.0f && end < far;
+                const float* q = lines + static_cast<int64_t>(k) * pitch;
+                const int64_t step = static_cast<int64_t>(dir) * pitch;
+                acc += inside ? lineSamples<false>(q, step, pos, R.sa, count, n)
+                              : lineSamples<true>(q, step, pos, R.sa, count, n);
+            }
+            sums[threadIdx.y * 32 + lane] = acc;
+            __syncthreads();
+            if (member == 0 && valid) {
+                for (int m = 1; m < perGroup; ++m)
+                    acc += sums[(threadIdx.y + m) * 32 + lane];
+                y[r] = R.len * acc;
+            }
+        }
+
+        // Adjoint. A warp owns a TILE x TILE tile (with a one-pixel halo) in shared memory for
+        // some views and splats 32 neighbouring rays at once, lane i delayed by i modulo m planes:
+        // on any plane, the lanes that add at the same step are m rays apart, and rays m apart are
+        // more than two pixels apart (the class check), so no two lanes touch one word and the
+        // tile needs no atomics. Taps outside the tile belong to the neighbouring tile (halo words
+        // are not written out). The NW warps of a block take views NW apart of the block's chunk;
+        // their tiles are added in warp order, the chunks' partial images in chunk order.
+        // Bound by the latency of the read-add-write chain of a step at 12 warps per SM (issue at
+        // 58 %, 28 instructions per step of 32 rays). 512^2 / 720 views / 730 pixels: 0.51 ms;
+        // eight warps sharing a tile, merging taps by shuffles and adding in phases, took 1.99.
+        template <int TILE>
+        struct Tile2d {
+            static constexpr int kPitch = TILE + 3; // odd: lanes along either axis spread over banks
+            static constexpr int kWords = kPitch * (TILE + 2);
+        };
+
+        template <int TILE, int G>
+        __device__ __forceinline__ void tileRays(float* acc, const JosephRay* __restrict__ rays,
+                                                 const float2* __restrict__ cps, int64_t nrays,
+                                                 const float* __restrict__ y, int64_t viewBase,
+                                                 int u, int u1, int m, int depth, int orgG, int orgA)
+        {
+            constexpr int kPitch = Tile2d<TILE>::kPitch;
+            constexpr int strG = G == 0 ? 1 : kPitch, strA = G == 0 ? kPitch : 1;
+            const int64_t r = viewBase + u;
             JosephRay R{};
             bool act = u <= u1;
             if (act)
                 R = rays[r];
-            act = act && R.n > 0 && (R.meta & 3) == G;
             int jLo = 0, jHi = -1;
-            if (act)
-                act = sampleRange(R, kLo, kHi, jLo, jHi);
+            act = act && R.n > 0 && (R.meta & 3) == G &&
+                  sampleRange(R, orgG, orgG + TILE - 1, jLo, jHi);
             const int dir = (R.meta & 4) ? -1 : 1;
-            float pa = 0.0f, pb = 0.0f, yl = 0.0f;
+            float pos = 0.0f, yl = 0.0f;
+            int off = 0; // planes from the tile's first plane in ray direction
             if (act) {
                 const int kFirst = R.k0 + jLo * dir;
-                const float2 cp = __ldg(cps + (floorDiv(kFirst, CPD) + 1) * nrays + r);
-                pa = cp.x, pb = cp.y;
+                pos = __ldg(cps + (kFirst / depth + 1) * nrays + r).x;
                 yl = __ldg(y + r) * R.len;
+                off = dir > 0 ? kFirst - orgG : orgG + TILE - 1 - kFirst;
             }
-            for (int dsel = 1; dsel >= -1; dsel -= 2) {
-                const bool part = act && dir == dsel;
+            const int late = u % m;
+            // rays towards higher and towards lower indices of a view cross planes in opposite
+            // order: one direction at a time
+            for (int d = 1; d >= -1; d -= 2) {
+                const bool part = act && dir == d;
                 if (!__any_sync(0xffffffffu, part))
                     continue;
-                // plane offsets t in ray order: k = kLo + t (dir > 0) or kHi - t (dir < 0)
-                const int kFirst = R.k0 + jLo * dir;
-                const int t0 = part ? (dsel > 0 ? kFirst - kLo : kHi - kFirst) : (1 << 20);
-                const int t1 = part ? t0 + (jHi - jLo) : -1;
-                int tMin = t0, tMax = t1;
-                for (int o = 16; o > 0; o >>= 1) {
-                    tMin = min(tMin, __shfl_xor_sync(0xffffffffu, tMin, o));
-                    tMax = max(tMax, __shfl_xor_sync(0xffffffffu, tMax, o));
-                }
-                for (int t = tMin; t <= tMax; ++t) {
-                    const bool on = part && t >= t0 && t <= t1;
-                    const int k = dsel > 0 ? kLo + t : kHi - t;
-                    float* plane = acc + (k - orgG) * AR::strG;
-                    int L = 0, O = 0;
-                    float A = 0.0f, B = 0.0f, C = 0.0f, D = 0.0f;
-                    if (on) {
-                        Weights w;
-                        tapWeights(pa, pb, w);
-                        const int la = w.ia - orgA, lb = w.ib - orgB;
-                        L = LB ? lb : la;
-                        O = DIM == 2 ? 0 : (LB ? la : lb);
-                        const float wl0 = LB ? w.wb : w.wa, wl1 = LB ? w.cwb : w.cwa;
-                        const float wo0 = LB ? w.wa : w.wb, wo1 = LB ? w.cwa : w.cwb;
-                        if (DIM == 2) {
-                            A = yl * wl0;
-                            B = yl * wl1;
-                        } else {
-                            A = yl * (wl0 * wo0);
-                            B = yl * (wl1 * wo0);
-                            C = yl * (wl0 * wo1);
-                            D = yl * (wl1 * wo1);
-                        }
-                        pa = __fadd_rn(pa, R.sa);
-                        pb = __fadd_rn(pb, R.sb);
-                    }
-                    // neighbour state packed in one word: bit 0 active, bits 1.. column + 2^20
-                    const int packed = on ? (((L + (1 << 20)) << 1) | 1) : 0;
-                    const int prev = __shfl_up_sync(0xffffffffu, packed, 1);
-                    const int prev2 = __shfl_up_sync(0xffffffffu, packed, 2);
-                    const bool pOn = lane > 0 && (prev & 1);
-                    const int pL = (prev >> 1) - (1 << 20);
-                    const bool p2On = lane > 1 && (prev2 & 1);
-                    const int p2L = (prev2 >> 1) - (1 << 20);
-                    const bool second = on && pOn && pL == L; // second ray on this column
-                    // columns must be monotone along the active lanes and hold at most two rays
-                    const bool inc = __any_sync(0xffffffffu, on && pOn && pL < L);
-                    const bool dec = __any_sync(0xffffffffu, on && pOn && pL > L);
-                    const bool triple = __any_sync(0xffffffffu, second && p2On && p2L == L);
-                    if (!(inc && dec) && !triple) {
-                        // first rays of distinct columns, then second rays: within one phase
-                        // all writers sit on distinct columns
-#pragma unroll
-                        for (int ph = 0; ph < 4; ++ph) {
-                            const bool mine = on && (second == (ph >= 2));
-                            const int col = L + (ph & 1);
-                            if (mine) {
-                                addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, col, O, (ph & 1) ? B : A);
-                                if (DIM == 3)
-                                    addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, col, O + 1,
-                                                                       (ph & 1) ? D : C);
-                            }
-                            __syncwarp();
-                        }
-                    } else {
-                        for (int ph = 0; ph < m; ++ph) {
-                            if (on && lane % m == ph) {
-                                addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, L, O, A);
-                                addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, L + 1, O, B);
-                                if (DIM == 3) {
-                                    addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, L, O + 1, C);
-                                    addTap<EXT_L, EXT_O, STR_L, STR_O>(plane, L + 1, O + 1, D);
-                                }
-                            }
-                            __syncwarp();
-                        }
-                    }
+                const int first = part ? off + late : 1 << 20;
+                const int last = part ? first + jHi - jLo : -1;
+                int t = __reduce_min_sync(0xffffffffu, first);
+                const int tEnd = __reduce_max_sync(0xffffffffu, last);
+                // byte address of the sample's left tap: base + column * 4 strA (the halo column
+                // is -1), less the bias of the floor's bit pattern
+                const int plane0 = (d > 0 ? t - late : TILE - 1 - (t - late)) + 1;
+                unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(acc)) +
+                                4u * static_cast<unsigned>(plane0 * strG + (1 - orgA) * strA) -
+                                0x4B400000u * 4u * strA;
+                const unsigned bias = 0x4B400000u + static_cast<unsigned>(orgA) - 1u;
+                const unsigned span = part ? static_cast<unsigned>(last - first) : 0u;
+                for (; t <= tEnd; ++t) {
+                    const float h = __fsub_rn(pos, 0.5f);
+                    const float f = __fadd_rd(h, 12582912.0f); // floorSmall
+                    const float cw = __fsub_rn(h, __fsub_rn(f, 12582912.0f));
+                    const unsigned on =
+                        part & (static_cast<unsigned>(t - first) <= span);
+                    const unsigned in =
+                        on & (__float_as_uint(f) - bias < static_cast<unsigned>(TILE + 1));
+                    const unsigned q = base + __float_as_uint(f) * (4u * strA);
+                    float a, b;
+                    loadSharedIf(a, q, in);
+                    loadSharedIf(b, q + 4u * strA, in);
+                    storeSharedIf(__fmaf_rn(yl, __fsub_rn(1.0f, cw), a), q, in);
+                    storeSharedIf(__fmaf_rn(yl, cw, b), q + 4u * strA, in);
+                    pos = on ? __fadd_rn(pos, R.sa) : pos;
+                    base += static_cast<unsigned>(4 * d * strG);
+                    __syncwarp();
                 }
             }
         }
 
-        // All row segments of one (view, driving axis G) for a brick. Warps take (row, 32-ray
-        // segment) units; units that run concurrently are rows at least m apart or segments
-        // separated by a whole segment, so their taps are disjoint. Phases end with barriers.
-        template <int DIM, int G, bool LB, int BX, int BY, int BZ, int CPD, int NW>
-        __device__ __forceinline__ void splatView(float* acc, const RayWindow& w, int p,
-                                                  const JosephRay* __restrict__ rays,
-                                                  const float2* __restrict__ cps, int64_t nrays,
-                                                  const float* __restrict__ y,
-                                                  const DetectorShape& det, int m, int org0,
-                                                  int org1, int org2)
-        {
-            const int orgG = G == 0 ? org0 : (G == 1 ? org1 : org2);
-            const int orgA = G == 0 ? org1 : org0;
-            const int orgB = DIM == 2 ? 0 : (G == 2 ? org1 : org2);
-            const int warp = threadIdx.x >> 5;
-            const int nseg = (w.u1 - w.u0) / 32 + 1;
-            const int rowPhases = DIM == 3 ? m : 1;
-            for (int pr = 0; pr < rowPhases; ++pr) {
-                const int vFirst = w.v0 + pr;
-                const int nRows = DIM == 3 ? (vFirst <= w.v1 ? (w.v1 - vFirst) / m + 1 : 0) : 1;
-                for (int ps = 0; ps < 2 && ps < nseg; ++ps) {
-                    const int nSegs = (nseg - ps + 1) / 2;
-                    const int units = nRows * nSegs;
-                    for (int unit = warp; unit < units; unit += NW) {
-                        const int row = unit / nSegs, seg = unit - row * nSegs;
-                        const int v = DIM == 3 ? vFirst + row * m : 0;
-                        splatRowSegment<DIM, G, LB, BX, BY, BZ, CPD>(
-                            acc, rays, cps, nrays, y, det, p, v, w.u0 + 32 * (ps + 2 * seg),
-                            w.u1, m, orgG, orgA, orgB);
-                    }
-                    __syncthreads();
-                }
-            }
-        }
-
-        // One CTA per brick of BX x BY x BZ voxels (BZ = 1 in 2D), NW warps. The brick
-        // accumulates every view in a fixed order and is written once.
-        template <int DIM, int BX, int BY, int BZ, int CPD, int NW>
+        template <int TILE, int NW>
         __global__ void __launch_bounds__(NW * 32)
-            josephAdjointKernel(const JosephRay* __restrict__ rays,
-                                const float2* __restrict__ checkpoints, int64_t nrays,
-                                const float* __restrict__ y,
-                                const RayWindow* __restrict__ windows,
-                                const unsigned* __restrict__ viewAxes, VolumeShape vol,
-                                DetectorShape det, int m, int3 nBricks, int viewsPerChunk,
-                                float* __restrict__ x)
+            josephAdjoint2dKernel(const JosephRay* __restrict__ rays,
+                                  const float2* __restrict__ checkpoints, int64_t nrays,
+                                  const float* __restrict__ y,
+                                  const RayWindow* __restrict__ windows,
+                                  const unsigned* __restrict__ viewAxes, VolumeShape vol,
+                                  DetectorShape det, int m, int depth, int2 tiles,
+                                  int viewsPerChunk, float* __restrict__ x)
         {
-            // blockIdx.y selects a chunk of views; with several chunks each CTA writes its
-            // partial brick to x + chunk * nvox and a second pass sums the chunks in order
+            // blockIdx.x: tile, blockIdx.y: view chunk (partial image x + chunk * nvox)
             extern __shared__ float smem[];
-            using L = BrickLayout<DIM, BX, BY>;
-            constexpr int NT = NW * 32;
-            constexpr int kWords = L::kPlane * BZ;
-            float* acc = smem;
-            RayWindow* win = reinterpret_cast<RayWindow*>(smem + ((kWords + 3) & ~3));
-            unsigned* axes = reinterpret_cast<unsigned*>(win + det.np);
-            const int bi = blockIdx.x;
-            const int org0 = (bi % nBricks.x) * BX, org1 = ((bi / nBricks.x) % nBricks.y) * BY,
-                      org2 = (bi / (nBricks.x * nBricks.y)) * BZ;
-            const int nb = nBricks.x * nBricks.y * nBricks.z;
+            constexpr int kWords = Tile2d<TILE>::kWords, kPitch = Tile2d<TILE>::kPitch;
+            const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+            float* acc = smem + warp * kWords;
+            const int org0 = (blockIdx.x % tiles.x) * TILE, org1 = (blockIdx.x / tiles.x) * TILE;
+            for (int i = lane; i < kWords; i += 32)
+                acc[i] = 0.0f;
+            __syncwarp();
             const int pBegin = blockIdx.y * viewsPerChunk;
             const int pEnd = min(det.np, pBegin + viewsPerChunk);
-            for (int i = threadIdx.x; i < kWords; i += NT)
-                acc[i] = 0.0f;
-            for (int p = pBegin + threadIdx.x; p < pEnd; p += NT) {
-                const RayWindow w = windows[static_cast<int64_t>(p) * nb + bi];
-                win[p] = w;
-                axes[p] = (w.u0 > w.u1 || w.v0 > w.v1) ? 0u : viewAxes[p];
+            const int64_t nTiles = static_cast<int64_t>(tiles.x) * tiles.y;
+            for (int p = pBegin + warp; p < pEnd; p += NW) {
+                const RayWindow w = windows[p * nTiles + blockIdx.x];
+                const unsigned axes = viewAxes[p];
+                const int64_t viewBase = static_cast<int64_t>(det.nu) * p;
+                for (int u = w.u0 + lane; u - lane <= w.u1; u += 32) {
+                    if (axes & 1u)
+                        tileRays<TILE, 0>(acc, rays, checkpoints, nrays, y, viewBase, u, w.u1, m,
+                                          depth, org0, org1);
+                    if (axes & 2u)
+                        tileRays<TILE, 1>(acc, rays, checkpoints, nrays, y, viewBase, u, w.u1, m,
+                                          depth, org1, org0);
+                }
             }
             __syncthreads();
-            const int64_t nvox = static_cast<int64_t>(vol.n[0]) * vol.n[1] * vol.n[2];
-            float* out = x + blockIdx.y * nvox;
-            for (int p = pBegin; p < pEnd; ++p) {
-                const unsigned ax = axes[p];
-                if (!(ax & 7u))
+            float* out = x + blockIdx.y * (static_cast<int64_t>(vol.n[0]) * vol.n[1]);
+            for (int i = threadIdx.x; i < TILE * TILE; i += NW * 32) {
+                const int lx = i % TILE, ly = i / TILE;
+                if (org0 + lx >= vol.n[0] || org1 + ly >= vol.n[1])
                     continue;
-                const RayWindow w = win[p];
-                // bit g: rays drive along g; bit 4+g: their lanes spread along axis b
-#define ELSA_SPLAT(G_)                                                                            \
-    if (ax & (1u << G_)) {                                                                        \
-        if (ax & (16u << G_))                                                                     \
-            splatView<DIM, G_, true, BX, BY, BZ, CPD, NW>(acc, w, p, rays, checkpoints, nrays, y, \
-                                                          det, m, org0, org1, org2);              \
-        else                                                                                      \
-            splatView<DIM, G_, false, BX, BY, BZ, CPD, NW>(acc, w, p, rays, checkpoints, nrays,   \
-                                                           y, det, m, org0, org1, org2);          \
-    }
-                ELSA_SPLAT(0)
-                ELSA_SPLAT(1)
-                if (DIM == 3) {
-                    ELSA_SPLAT((DIM == 3 ? 2 : 1))
-                }
-#undef ELSA_SPLAT
-            }
-            for (int i = threadIdx.x; i < BX * BY * BZ; i += NT) {
-                const int lx = i % BX, ly = (i / BX) % BY, lz = i / (BX * BY);
-                const int gx = org0 + lx, gy = org1 + ly, gz = org2 + lz;
-                if (gx < vol.n[0] && gy < vol.n[1] && gz < vol.n[2])
-                    out[gx + static_cast<int64_t>(vol.n[0]) *
-                                 (gy + static_cast<int64_t>(vol.n[1]) * gz)] =
-                        acc[lz * L::kPlane + ly * L::kRow + lx];
+                const float* q = smem + (ly + 1) * kPitch + lx + 1;
+                float s = q[0];
+                for (int k = 1; k < NW; ++k)
+                    s = s + q[k * kWords];
+                out[org0 + lx + static_cast<int64_t>(vol.n[0]) * (org1 + ly)] = s;
             }
         }
 
@@ -923,10 +855,6 @@ namespace elsa_b200
             }
         }
 
-#ifndef ELSA_ADJ2D_CTAS_PER_SM
-#define ELSA_ADJ2D_CTAS_PER_SM 16
-#endif
-        constexpr int kAdjoint2dCtasPerSm = ELSA_ADJ2D_CTAS_PER_SM;
 #ifndef ELSA_ADJ3D_WARPS_PER_SM
 #define ELSA_ADJ3D_WARPS_PER_SM 22
 #endif
@@ -935,60 +863,38 @@ namespace elsa_b200
         constexpr int64_t kChunkMemory = int64_t(1) << 31;   // default partial-volume budget
         constexpr int64_t kBatchPartialMemory = int64_t(8) << 30; // batched adjoints: up to 8 GiB
 
-        template <int DIM, int BX, int BY, int BZ, int CPD, int NW>
-        struct AdjointConfig {
-            using L = BrickLayout<DIM, BX, BY>;
-            static constexpr size_t kAccBytes = sizeof(float) * ((L::kPlane * BZ + 3) & ~3);
-            static constexpr int kThreads = NW * 32;
-            static constexpr int kCheckpointDepth = CPD;
-            static_assert(BX % CPD == 0 && BY % CPD == 0 && (DIM == 2 || BZ % CPD == 0),
-                          "brick edges must be multiples of the checkpoint depth");
-            static int3 brick() { return make_int3(BX, BY, BZ); }
-            // accumulator + per-view windows and axis masks
-            static size_t smemBytes(int np)
+        template <int TILE, int NW>
+        struct Adjoint2dConfig {
+            static constexpr size_t kShared = sizeof(float) * Tile2d<TILE>::kWords * NW;
+            static constexpr int kBlocksPerSm = static_cast<int>((227 * 1024) / (kShared + 1024));
+            // View chunks so that tiles x chunks is one wave of blocks, each warp with a view.
+            static int chunks(int tiles, int np)
             {
-                return kAccBytes + (sizeof(RayWindow) + sizeof(unsigned)) * np;
+                const int want = (kBlocksPerSm * 148 + tiles - 1) / tiles;
+                return std::max(1, std::min(want, (np + NW - 1) / NW));
             }
-            // The dynamic shared-memory limit is an attribute of the kernel on the device, shared
-            // by every projector: it only ever grows, so a projector with fewer views created
-            // later leaves room for the earlier ones.
-            static void prepare(int np)
+            static void prepare()
             {
-                static std::mutex mu;
-                std::lock_guard<std::mutex> lock(mu);
-                cudaFuncAttributes attr{};
-                ELSA_CUDA(cudaFuncGetAttributes(&attr,
-                                                josephAdjointKernel<DIM, BX, BY, BZ, CPD, NW>));
-                const int need = static_cast<int>(smemBytes(np));
-                if (need > attr.maxDynamicSharedSizeBytes)
-                    ELSA_CUDA(cudaFuncSetAttribute(josephAdjointKernel<DIM, BX, BY, BZ, CPD, NW>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   need));
+                ELSA_CUDA(cudaFuncSetAttribute(josephAdjoint2dKernel<TILE, NW>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kShared)));
             }
-            // Views per chunk so that bricks x chunks fills about kAdjoint2dCtasPerSm CTAs per SM
-            // (16 measured best among 1-16 at 128^2 x 180 views and 512^2 x 720 views). The
-            // partial volumes then hold fewer than 2 x 16 x 148 tiles of 64 x 64 floats (78 MB).
-            static int chunks(int nbricks, int np)
-            {
-                const int want = (kAdjoint2dCtasPerSm * 148 + nbricks - 1) / nbricks;
-                return want < 1 ? 1 : (want > np ? np : want);
-            }
-            // nc view chunks; partial: scratch of nc volumes (unused with one chunk)
-            static void launch(int nbricks, int nc, cudaStream_t s, const JosephRay* rays,
+            // nc view chunks; partial: scratch of nc images (unused with one chunk)
+            static void launch(int2 tiles, int nc, int depth, cudaStream_t s, const JosephRay* rays,
                                const float2* cps, int64_t nrays, const float* y,
                                const RayWindow* win, const unsigned* axes, VolumeShape vol,
-                               DetectorShape det, int m, int3 nb, float* x, float* partial)
+                               DetectorShape det, int m, float* x, float* partial)
             {
                 const int per = (det.np + nc - 1) / nc;
                 const int used = (det.np + per - 1) / per;
-                const dim3 grid(static_cast<unsigned>(nbricks), static_cast<unsigned>(used));
-                josephAdjointKernel<DIM, BX, BY, BZ, CPD, NW>
-                    <<<grid, kThreads, smemBytes(det.np), s>>>(rays, cps, nrays, y, win, axes,
-                                                               vol, det, m, nb, per,
-                                                               used > 1 ? partial : x);
+                const dim3 grid(static_cast<unsigned>(tiles.x * tiles.y),
+                                static_cast<unsigned>(used));
+                josephAdjoint2dKernel<TILE, NW><<<grid, NW * 32, kShared, s>>>(
+                    rays, cps, nrays, y, win, axes, vol, det, m, depth, tiles, per,
+                    used > 1 ? partial : x);
                 if (used > 1)
                     launchSumChunks(partial, used,
-                                    static_cast<int64_t>(vol.n[0]) * vol.n[1] * vol.n[2], x, s);
+                                    static_cast<int64_t>(vol.n[0]) * vol.n[1], x, s);
             }
         };
 
@@ -1308,7 +1214,11 @@ namespace elsa_b200
                                                   static_cast<int>(local / nb), acc);
         }
 
-        using Adjoint2d = AdjointConfig<2, 64, 64, 1, 64, 8>;
+        // Tiles of 64 pixels for images that fill the GPU with them, of 32 for smaller ones (more
+        // blocks; their rays start and end in more tiles).
+        using Adjoint2dLarge = Adjoint2dConfig<64, 4>;
+        using Adjoint2dSmall = Adjoint2dConfig<32, 8>;
+                constexpr int kSmallImage = 256 * 256; // pixels (512^2: 0.504 ms with tiles of 32, 0.514 of 64)
 
         class JosephProjector final : public Projector
         {
@@ -1350,6 +1260,8 @@ namespace elsa_b200
                         classSpacing_ = m;
                         break;
                     }
+                if (vol_.dim == 2)
+                    buildForward2d();
                 if (fast_) {
                     buildFastAdjoint();
                     if (vol_.dim == 3) {
@@ -1367,15 +1279,12 @@ namespace elsa_b200
                                 "of each other even eight pixels apart; the atomic-free adjoint "
                                 "needs a coarser detector");
 
-                int cpd;
                 if (vol_.dim == 3) {
-                    cpd = defaultCheckpointDepth();
+                    buildCheckpoints(defaultCheckpointDepth());
                 } else {
-                    brick_ = Adjoint2d::brick();
-                    cpd = Adjoint2d::kCheckpointDepth;
-                    Adjoint2d::prepare(det_.np);
+                    Adjoint2dLarge::prepare();
+                    Adjoint2dSmall::prepare();
                 }
-                buildCheckpoints(cpd);
 
                 if (vol_.dim == 3) {
                     buildAxisGrids();
@@ -1399,6 +1308,20 @@ namespace elsa_b200
                 }
                 ELSA_CUDA(cudaDeviceSynchronize());
                 curved_.release(); // rays and windows are built
+            }
+
+            // 2D: checkpoints, one slab per tile of the adjoint, and the padded image copies.
+            void buildForward2d()
+            {
+                const int tile = domainSize_ <= kSmallImage ? 32 : 64;
+                brick_ = make_int3(tile, tile, 1);
+                buildCheckpoints(tile);
+                rows_ = std::make_unique<DeviceBuffer>(sizeof(float) * vol_.n[1] *
+                                                       linePitch(vol_.n[0]));
+                columns_ = std::make_unique<DeviceBuffer>(sizeof(float) * vol_.n[0] *
+                                                          linePitch(vol_.n[1]));
+                ELSA_CUDA(cudaMemset(rows_->as<float>(), 0, rows_->bytes()));
+                ELSA_CUDA(cudaMemset(columns_->as<float>(), 0, columns_->bytes()));
             }
 
             // Per view and driving axis g: set bit 4+g of the view's axis word when neighbouring
@@ -1526,18 +1449,35 @@ namespace elsa_b200
 
             void forward(const float* x, float* y, cudaStream_t s) override
             {
-                const int64_t nrays = rangeSize_;
-                const unsigned blocks =
-                    static_cast<unsigned>((nrays + forwardThreads_ - 1) / forwardThreads_);
                 if (tma_)
                     tma_->forward(x, y, s);
-                else if (vol_.dim == 3)
-                    josephForwardKernel<3><<<blocks, forwardThreads_, 0, s>>>(dRays_, nrays, x,
-                                                                                vol_, y);
                 else
-                    josephForwardKernel<2><<<blocks, forwardThreads_, 0, s>>>(dRays_, nrays, x,
-                                                                                vol_, y);
-                ELSA_LAUNCH_CHECK("josephForwardKernel");
+                    forward2d(x, y, s);
+            }
+
+            void forward2d(const float* x, float* y, cudaStream_t s)
+            {
+                const dim3 blocks((vol_.n[0] + 31) / 32, (vol_.n[1] + 31) / 32);
+                padLinesKernel<<<blocks, dim3(32, 8), 0, s>>>(
+                    x, vol_.n[0], vol_.n[1], rows_->as<float>(), columns_->as<float>());
+                ELSA_LAUNCH_CHECK("padLinesKernel");
+                const int depth = 1 << cpdShift_;
+                const int slabs = (std::max(vol_.n[0], vol_.n[1]) + depth - 1) / depth;
+                const int segments = (det_.nu + 31) / 32;
+                const int warps = forwardThreads_ / 32;
+                // warps per view segment: as many as fill 32 warps per SM, at most its slabs
+                int perGroup = 1;
+                while (2 * perGroup <= std::min(warps, slabs) &&
+                       static_cast<int64_t>(segments) * det_.np * perGroup < 148 * 32)
+                    perGroup *= 2;
+                const int groups = warps / perGroup;
+                const int64_t grid =
+                    static_cast<int64_t>(segments) * ((det_.np + groups - 1) / groups);
+                josephForward2dKernel<<<static_cast<unsigned>(grid), dim3(32, groups * perGroup), 0,
+                                        s>>>(dRays_, dCheckpoints_, rangeSize_, vol_, det_, depth,
+                                             slabs, groups, segments, rows_->as<float>(),
+                                             columns_->as<float>(), y);
+                ELSA_LAUNCH_CHECK("josephForward2dKernel");
             }
 
             void adjoint(const float* y, float* x, cudaStream_t s) override
@@ -1589,12 +1529,12 @@ namespace elsa_b200
                         launchSumChunks(partial_->as<float>(), axisPartials_, domainSize_, x, s);
                     return;
                 }
-                const int nb = nBricks_.x * nBricks_.y * nBricks_.z;
                 float* partial = partial_ ? partial_->as<float>() : nullptr;
-                Adjoint2d::launch(nb, adjointChunks_, s, dRays_, dCheckpoints_, rangeSize_, y,
-                                  dWindows_, dViewAxes_, vol_, det_, classSpacing_, nBricks_, x,
-                                  partial);
-                ELSA_LAUNCH_CHECK("josephAdjointKernel");
+                auto* launch = brick_.x == 64 ? Adjoint2dLarge::launch : Adjoint2dSmall::launch;
+                launch(make_int2(nBricks_.x, nBricks_.y), adjointChunks_, 1 << cpdShift_, s, dRays_,
+                       dCheckpoints_, rangeSize_, y, dWindows_, dViewAxes_, vol_, det_,
+                       classSpacing_, x, partial);
+                ELSA_LAUNCH_CHECK("josephAdjoint2dKernel");
             }
 
             // Batched applies (3D matched operator): one launch per kernel for all volumes,
@@ -1856,7 +1796,7 @@ namespace elsa_b200
                 case 4: // parts per million of detector tiles on the gather fallback
                     return tma_ ? static_cast<int64_t>(tma_->fallbackFraction() * 1e6) : -1;
                 case 6: // kernel launches per forward call
-                    return tma_ ? tma_->launchesPerForward() : 1;
+                    return tma_ ? tma_->launchesPerForward() : 2;
                 case 7: // kernel launches per adjoint call (3D: one per axis grid; with
                         // several partial volumes: + the chunk sum)
                     if (fast_ || scatter_)
@@ -1907,11 +1847,12 @@ namespace elsa_b200
             cudaTextureObject_t fastTex_ = 0;
             std::unique_ptr<DeviceBuffer> fastTable_;
             int scatter_ = 0; // 1: atomic scatter adjoint (2D: 512^2 / 720 views 1.74 ms
-                              // against 2.00; 3D 256^3 / 360 views 92 ms against 54.8)
+                              // against 0.51; 3D 256^3 / 360 views 92 ms against 28.2)
             JosephRay* dRays_ = nullptr;
             unsigned* dViewAxes_ = nullptr;
             RayWindow* dWindows_ = nullptr;
             float2* dCheckpoints_ = nullptr;
+            std::unique_ptr<DeviceBuffer> rows_, columns_; // 2D: the forward's padded image copies
             int cpStride_ = 0;
             int cpdShift_ = 4; // checkpoint slabs of 2^cpdShift_ planes (3D)
 
@@ -1936,7 +1877,8 @@ namespace elsa_b200
             {
                 int fill;
                 if (vol_.dim == 2) {
-                    fill = Adjoint2d::chunks(nBricks_.x * nBricks_.y * nBricks_.z, det_.np);
+                    fill = brick_.x == 64 ? Adjoint2dLarge::chunks(nBricks_.x * nBricks_.y, det_.np)
+                                          : Adjoint2dSmall::chunks(nBricks_.x * nBricks_.y, det_.np);
                 } else {
                     // bricks x chunks of the smallest present grid reach kAdjoint3dWarpsPerSm
                     // one-warp CTAs per SM (each grid sees about its share of the views)
@@ -1952,8 +1894,9 @@ namespace elsa_b200
                 // axis grid) pair, so leave room for the chunks whose views drive along two axes
                 const int64_t cap = std::max<int64_t>(1, kChunkMemory / (4 * domainSize_));
                 const int64_t capChunks = vol_.dim == 3 ? std::max<int64_t>(1, cap * 7 / 8) : cap;
-                return static_cast<int>(std::min<int64_t>(
-                    std::min<int64_t>(det_.np, capChunks), std::max(fill, kMinAdjointChunks)));
+                const int least = vol_.dim == 3 ? kMinAdjointChunks : 1;
+                return static_cast<int>(std::min<int64_t>(std::min<int64_t>(det_.np, capChunks),
+                                                          std::max(fill, least)));
             }
 
             // ---- 3D matched adjoint on axis bricks ----

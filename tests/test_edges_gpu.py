@@ -31,6 +31,39 @@ def _problem(oracle, vol, views, det, arc=360, seed=3):
     return poses, det, x, y
 
 
+@pytest.mark.parametrize("vol,views,det", [
+    ((1, 1), 3, [3]), ((31, 33), 5, [31]), ((32, 32), 7, [33]), ((65, 40), 9, [64]),
+    ((127, 1), 4, [140]), ((256, 257), 6, [321]), ((300, 290), 11, [401]), ((1, 70), 8, [97])])
+def test_joseph_2d_tiles(cuda, oracle, vol, views, det):
+    """Tiles of 32 and 64 pixels, remainders, one-pixel edges; views around 45 degrees mix both
+    driving axes."""
+    import elsa_b200
+    poses, det, x, y = _problem(oracle, vol, views, det)
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, poses)
+    for threads in (64, 256, 512):
+        proj.set_knob(elsa_b200.KNOB_FORWARD_THREADS, threads)
+        assert rel_l2(_apply(cuda, proj, x, False), oracle.joseph(x, vol, det, poses)) <= PARITY
+    ref = oracle.joseph_adjoint(y, vol, det, poses)
+    first = _apply(cuda, proj, y, True)
+    assert rel_l2(first, ref) <= PARITY
+    assert np.array_equal(first, _apply(cuda, proj, y, True))
+    proj.set_knob(elsa_b200.KNOB_ADJOINT_CHUNKS, 1)
+    assert rel_l2(_apply(cuda, proj, y, True), ref) <= PARITY
+
+
+def test_joseph_2d_non_finite(cuda, oracle):
+    """An infinity reaches exactly the pixels whose rays meet it, as in the oracle."""
+    import elsa_b200
+    vol = (40, 37)
+    poses, det, x, _ = _problem(oracle, vol, 6, [50])
+    x[20 + 40 * 11] = np.inf
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, poses)
+    got = _apply(cuda, proj, x, False)
+    ref = np.asarray(oracle.joseph(x, vol, det, poses))
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref))
+    assert np.array_equal(np.isinf(got), np.isinf(ref))
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("kind,params", [
     ("blob", (2.0, 10.83, 2)), ("blob", (0.55, 10.83, 2)), ("blob", (3.7, 8.0, 1)),
