@@ -10,7 +10,7 @@
 // (projectors/JosephsMethod.cpp:60-97). Box origins per (tile, chunk) are computed once per
 // geometry from the same accumulated sample positions the kernel uses, so every tap is inside its
 // box; tiles whose rays disagree on axis or direction, or do not fit the box, use the per-ray
-// gather (the same arithmetic as josephForwardKernel).
+// gather.
 //
 // All waits on mbarriers are bounded (about one second of clock cycles by default); on timeout the
 // CTA records bit 0 of the error word, waits (bounded again) for the copies it has issued and
@@ -143,30 +143,47 @@ namespace elsa_b200
                 : "memory");
         }
 
-        // out[(k * nSlow + s) * padFast + f] = x(axis values), zero in the padding columns.
-        // blockIdx.y: batch element (x + b xStride into copy b of out)
-        __global__ void permuteKernel(const float* __restrict__ x, VolumeShape vol, int g, int sAx,
-                                      int fAx, int padFast, float* __restrict__ out,
-                                      int64_t xStride)
+        // A volume with another axis contiguous: out[sum of coordinate * outStride] = x. fast: the
+        // axis that is contiguous in out (outStride 1). 32 x 8 threads per 32 x 32 block of the
+        // (x, fast) plane, staged in shared memory so that reads and writes are both coalesced
+        // (256^3 forward: 10.51 ms reading along `fast` directly, 10.41 so); fast == x is a
+        // strided copy of rows. blockIdx.z counts the planes (and batch elements) in turn.
+        struct LayoutCopy {
+            int nx, nf, no, batch;
+            int64_t strF, strO;          // words of x per step along fast and the third axis
+            int64_t outX, outF, outO;    // words of out per step along x, fast and the third axis
+            int64_t xBatch, outBatch;
+        };
+
+        __global__ void __launch_bounds__(256)
+            layoutCopyKernel(const float* __restrict__ x, LayoutCopy c, float* __restrict__ out)
         {
-            const int nf = vol.n[fAx], ns = vol.n[sAx], ng = vol.n[g];
-            const int64_t total = static_cast<int64_t>(padFast) * ns * ng;
-            x += blockIdx.y * xStride;
-            out += blockIdx.y * total;
-            const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-            for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-                 i < total; i += stride) {
-                const int f = static_cast<int>(i % padFast);
-                const int s = static_cast<int>((i / padFast) % ns);
-                const int k = static_cast<int>(i / (static_cast<int64_t>(padFast) * ns));
-                float v = 0.0f;
-                if (f < nf) {
-                    int c[3];
-                    c[g] = k, c[sAx] = s, c[fAx] = f;
-                    v = __ldg(x + c[0] + static_cast<int64_t>(vol.n[0]) *
-                                             (c[1] + static_cast<int64_t>(vol.n[1]) * c[2]));
+            __shared__ float t[32][33];
+            const int x0 = blockIdx.x * 32, f0 = blockIdx.y * 32;
+            const int planes = c.no * c.batch;
+            for (int plane = blockIdx.z; plane < planes; plane += gridDim.z) {
+                const int b = plane / c.no, o = plane - b * c.no;
+                const float* src = x + b * c.xBatch + o * c.strO;
+                float* dst = out + b * c.outBatch + o * c.outO;
+                const int ix = x0 + threadIdx.x;
+                for (int j = threadIdx.y; j < 32; j += 8) {
+                    const int f = f0 + j;
+                    if (ix < c.nx && f < c.nf) {
+                        const float v = __ldg(src + ix + f * c.strF);
+                        if (c.outX == 1)
+                            dst[ix + f * c.outF] = v;
+                        else
+                            t[j][threadIdx.x] = v;
+                    }
                 }
-                out[i] = v;
+                if (c.outX == 1)
+                    continue;
+                __syncthreads();
+                const int f = f0 + threadIdx.x;
+                for (int j = threadIdx.y; j < 32; j += 8)
+                    if (x0 + j < c.nx && f < c.nf)
+                        dst[(x0 + j) * c.outX + f * c.outF] = t[threadIdx.x][j];
+                __syncthreads();
             }
         }
 
@@ -282,7 +299,7 @@ namespace elsa_b200
             }
         }
 
-        // The per-ray gather (fallback tiles): the arithmetic of josephForwardKernel.
+        // The per-ray gather (fallback tiles).
         __device__ float gatherRay(const JosephRay& R, const float* __restrict__ x,
                                    const VolumeShape& vol)
         {
@@ -534,9 +551,30 @@ namespace elsa_b200
             return fn;
         }
 
-        // Non-driving axis along which neighbouring pixels of a detector row spread, voted over
-        // the views (centre pixel and its right neighbour).
-        std::array<int, 3> fastAxes(const std::vector<float>& poses, const DetectorShape& det)
+    } // namespace
+
+    void launchLayoutCopy(const float* x, const VolumeShape& vol, int fast,
+                          const int64_t (&outStride)[3], float* out, cudaStream_t s, int batch,
+                          int64_t xStride, int64_t outBatchStride)
+    {
+        // with fast == x, the second axis takes the place of `fast` in the (x, fast) plane
+        const int f = fast == 0 ? 1 : fast, o = 3 - f;
+        const int64_t str[3] = {1, vol.n[0], static_cast<int64_t>(vol.n[0]) * vol.n[1]};
+        LayoutCopy c;
+        c.nx = vol.n[0], c.nf = vol.n[f], c.no = vol.n[o], c.batch = batch;
+        c.strF = str[f], c.strO = str[o];
+        c.outX = outStride[0], c.outF = outStride[f], c.outO = outStride[o];
+        c.xBatch = xStride, c.outBatch = outBatchStride;
+        const int64_t planes = static_cast<int64_t>(c.no) * batch;
+        const dim3 grid((c.nx + 31) / 32, (c.nf + 31) / 32,
+                        static_cast<unsigned>(std::min<int64_t>(planes, 65535)));
+        layoutCopyKernel<<<grid, dim3(32, 8), 0, s>>>(x, c, out);
+        ELSA_LAUNCH_CHECK("layoutCopyKernel");
+    }
+
+    // centre pixel and its right neighbour of every view
+    std::array<int, 3> fastAxes(const std::vector<float>& poses, const DetectorShape& det)
+    {
         {
             int votes[3][3] = {};
             for (int p = 0; p < det.np; ++p) {
@@ -565,7 +603,7 @@ namespace elsa_b200
             }
             return fast;
         }
-    } // namespace
+    }
 
     JosephForwardTma::JosephForwardTma(const VolumeShape& vol, const DetectorShape& det,
                                        const std::vector<float>& poses, const JosephRay* dRays)
@@ -681,9 +719,13 @@ namespace elsa_b200
         for (int g = 0; g < 3; ++g) {
             if (!present_[g])
                 continue;
-            permuteKernel<<<dim3(148 * 8, static_cast<unsigned>(batch)), 256, 0, s>>>(
-                x, vol_, g, slow_[g], fast_[g], padFast_[g], dLayouts_[g], xStride);
-            ELSA_LAUNCH_CHECK("permuteKernel");
+            // [g][slow][fast], rows padded to 16 bytes (the padding is outside the tensor map)
+            int64_t stride[3];
+            stride[fast_[g]] = 1;
+            stride[slow_[g]] = padFast_[g];
+            stride[g] = static_cast<int64_t>(padFast_[g]) * vol_.n[slow_[g]];
+            launchLayoutCopy(x, vol_, fast_[g], stride, dLayouts_[g], s, batch, xStride,
+                             stride[g] * vol_.n[g]);
         }
     }
 

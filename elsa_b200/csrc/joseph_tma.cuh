@@ -21,6 +21,16 @@ namespace elsa_b200
         int pad;
     };
 
+    // Per driving axis, the non-driving axis along which neighbouring pixels of a detector row
+    // spread, voted over the views (3D; poses as 40-float records).
+    std::array<int, 3> fastAxes(const std::vector<float>& poses, const DetectorShape& det);
+
+    // out[c0 outStride[0] + c1 outStride[1] + c2 outStride[2]] = x(c0, c1, c2) with
+    // outStride[fast] = 1, for `batch` volumes x + b xStride -> out + b outBatchStride.
+    void launchLayoutCopy(const float* x, const VolumeShape& vol, int fast,
+                          const int64_t (&outStride)[3], float* out, cudaStream_t s,
+                          int batch = 1, int64_t xStride = 0, int64_t outBatchStride = 0);
+
     class JosephForwardTma
     {
     public:
