@@ -26,11 +26,13 @@
 // each lane replays one ray's visits inside the slab from its checkpoint and adds the weights of
 // the visits that fall inside the brick. Same-class rays therefore never touch the same voxel,
 // and every voxel sums its contributions in a fixed order.
+#include "joseph_tma.cuh"
 #include "projector.hpp"
 #include "raysetup.cuh"
 #include "solvers.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cfloat>
 #include <climits>
 #include <cstring>
@@ -78,6 +80,28 @@ namespace elsa_b200
             return tm;
         }
 
+        // One axis of a visit: where its T is the crossing parameter, T, the word offset and the
+        // steps left advance, all predicated (the compiler selects and adds instead: 37
+        // instructions per visit against 27).
+        __device__ __forceinline__ void crossIf(float tm, float& T, float tDelta, unsigned& idx,
+                                                unsigned step, int& left, int one)
+        {
+            asm("{\n\t.reg .pred m;\n\tsetp.eq.f32 m, %0, %3;\n\t"
+                "@m add.rn.f32 %0, %0, %4;\n\t@m add.u32 %1, %1, %5;\n\t"
+                "@m sub.s32 %2, %2, %6;\n\t}"
+                : "+f"(T), "+r"(idx), "+r"(left)
+                : "f"(tm), "f"(tDelta), "r"(step), "r"(one));
+        }
+        __device__ __forceinline__ void crossIf(float tm, float& T, float tDelta, int64_t& idx,
+                                                int64_t step, int& left, int one)
+        {
+            if (T == tm) {
+                left -= one;
+                idx += step;
+                T = __fadd_rn(T, tDelta);
+            }
+        }
+
         // Entry voxel in axis order from the record (g and the two other axes a < b).
         __device__ __forceinline__ void entryVoxel(int g, int kg, int ca, int cb, int& c0,
                                                    int& c1, int& c2)
@@ -87,10 +111,25 @@ namespace elsa_b200
             c2 = g == 2 ? kg : cb;
         }
 
-        template <int DIM>
+        // Per driving axis of a ray, the copy of the volume it is read from (the volume itself, or
+        // one with the axis contiguous along which neighbouring rays spread) and its strides.
+        struct SiddonLayouts {
+            const float* base[3];
+            int64_t stride[3][3];
+        };
+
+        // One thread per ray, the reference's visits and float operations in order. Bound by issue
+        // (about 25 instructions per visit) once neighbouring lanes read neighbouring words: with
+        // every ray on the x-fastest volume, a warp whose rays drive along x read 32 sectors per
+        // visit and the load pipe took the time (171 x 200 x 149 voxels, 240 views of
+        // 250 x 231: 3.62 ms, now 2.69). The bounds test counts the steps left along each axis, so a visit updates
+        // one word offset instead of three voxel indices and a 64-bit one. Offset: unsigned below
+        // 2^32 words, else int64_t.
+        template <int DIM, typename Offset>
         __global__ void __launch_bounds__(kMaxForwardThreads)
             siddonForwardKernel(const SiddonRay* __restrict__ rays, int64_t nrays,
-                                const float* __restrict__ x, VolumeShape vol, int binary,
+                                const __grid_constant__ SiddonLayouts layouts, VolumeShape vol,
+                                int binary,
                                 float* __restrict__ y)
         {
             // binary: BinaryMethod (projectors/BinaryMethod.cpp:66-111), weight 1 per visit
@@ -105,37 +144,32 @@ namespace elsa_b200
                 entryVoxel(g, R.kFirst, R.cur[0], R.cur[1], c0, c1, c2);
                 const int s0 = axisStep(R.meta, 0), s1 = axisStep(R.meta, 1),
                           s2 = axisStep(R.meta, 2);
-                const int nx = vol.n[0], ny = vol.n[1], nz = vol.n[2];
-                const int64_t sy = nx, sz = static_cast<int64_t>(nx) * ny;
-                int64_t idx = c0 + sy * c1 + (DIM == 3 ? sz * c2 : 0);
+                const float* base = layouts.base[g];
+                const Offset e0 = static_cast<Offset>(layouts.stride[g][0]),
+                             e1 = static_cast<Offset>(layouts.stride[g][1]),
+                             e2 = DIM == 3 ? static_cast<Offset>(layouts.stride[g][2]) : 0;
+                Offset idx = c0 * e0 + c1 * e1 + (DIM == 3 ? c2 * e2 : 0);
+                const Offset i0 = s0 * e0, i1 = s1 * e1, i2 = s2 * e2;
+                // steps left before the ray leaves the volume (the entry voxel is inside)
+                int left0 = s0 > 0 ? vol.n[0] - 1 - c0 : c0;
+                int left1 = s1 > 0 ? vol.n[1] - 1 - c1 : c1;
+                int left2 = DIM == 3 ? (s2 > 0 ? vol.n[2] - 1 - c2 : c2) : 0;
+                const int k0 = s0 != 0, k1 = s1 != 0, k2 = s2 != 0;
                 float T0 = R.T[0], T1 = R.T[1], T2 = R.T[2];
                 float tExit = 0.0f;
-                const int maxVisits = nx + ny + (DIM == 3 ? nz : 0) + 3;
+                const int maxVisits = vol.n[0] + vol.n[1] + (DIM == 3 ? vol.n[2] : 0) + 3;
                 for (int it = 0; it < maxVisits; ++it) {
+                    const float v = __ldg(base + idx);
                     const float tEntry = tExit;
-                    bool m0, m1, m2;
-                    tExit = nextCrossing<DIM>(T0, T1, T2, m0, m1, m2);
-                    if (m0) {
-                        c0 += s0;
-                        T0 = __fadd_rn(T0, R.tDelta[0]);
-                    }
-                    if (m1) {
-                        c1 += s1;
-                        T1 = __fadd_rn(T1, R.tDelta[1]);
-                    }
-                    if (m2) {
-                        c2 += s2;
-                        T2 = __fadd_rn(T2, R.tDelta[2]);
-                    }
-                    const bool inside =
-                        static_cast<unsigned>(c0) < static_cast<unsigned>(nx) &&
-                        static_cast<unsigned>(c1) < static_cast<unsigned>(ny) &&
-                        (DIM < 3 || static_cast<unsigned>(c2) < static_cast<unsigned>(nz));
+                    tExit = DIM == 3 ? fminf(T0, fminf(T1, T2)) : fminf(T0, T1);
+                    crossIf(tExit, T0, R.tDelta[0], idx, i0, left0, k0);
+                    crossIf(tExit, T1, R.tDelta[1], idx, i1, left1, k1);
+                    if (DIM == 3)
+                        crossIf(tExit, T2, R.tDelta[2], idx, i2, left2, k2);
                     const float w = binary ? 1.0f : __fsub_rn(tExit, tEntry);
-                    acc = __fadd_rn(acc, __fmul_rn(__ldg(x + idx), w));
-                    if (!inside)
+                    acc = __fadd_rn(acc, __fmul_rn(v, w));
+                    if ((left0 | left1 | left2) < 0)
                         break;
-                    idx += (m0 ? s0 : 0) + (m1 ? s1 * sy : 0) + (m2 ? s2 * sz : 0);
                 }
             }
             y[r] = acc;
@@ -864,6 +898,7 @@ namespace elsa_b200
                         classSpacing_ = m;
                         break;
                     }
+                chooseLayouts();
                 const int bz = vol_.dim == 3 ? kSlab : 1;
                 nBricks_ = make_int3((vol_.n[0] + kSlab - 1) / kSlab,
                                      (vol_.n[1] + kSlab - 1) / kSlab, (vol_.n[2] + bz - 1) / bz);
@@ -883,17 +918,72 @@ namespace elsa_b200
                 ELSA_CUDA(cudaDeviceSynchronize());
             }
 
+            // The axis that is contiguous in the volume each driving axis is read from, and the
+            // copies' buffers (for the driving axes that occur).
+            void chooseLayouts()
+            {
+                std::vector<unsigned> axes(static_cast<size_t>(det_.np));
+                ELSA_CUDA(cudaMemcpy(axes.data(), viewAxes_->as<unsigned>(),
+                                     sizeof(unsigned) * axes.size(), cudaMemcpyDeviceToHost));
+                unsigned present = 0;
+                for (unsigned a : axes)
+                    present |= a;
+                if (vol_.dim == 3) {
+                    std::vector<float> hp(poses_.size() * kPoseFloats);
+                    std::memcpy(hp.data(), poses_.data(), sizeof(float) * hp.size());
+                    fast_ = fastAxes(hp, det_);
+                } else {
+                    fast_ = {1, 0, 0};
+                }
+                for (int g = 0; g < vol_.dim; ++g) {
+                    const int f = fast_[g];
+                    if (!((present >> g) & 1u)) {
+                        fast_[g] = 0;
+                    } else if (f != 0 && !copies_[f]) {
+                        try {
+                            copies_[f] = std::make_unique<DeviceBuffer>(
+                                sizeof(float) * static_cast<size_t>(domainSize_));
+                        } catch (const Error&) { // no room: the volume itself serves
+                            cudaGetLastError();
+                            fast_[g] = 0;
+                        }
+                    }
+                }
+            }
+
             void forward(const float* x, float* y, cudaStream_t s) override
             {
                 const int64_t nrays = rangeSize_;
                 const unsigned blocks =
                     static_cast<unsigned>((nrays + forwardThreads_ - 1) / forwardThreads_);
-                if (vol_.dim == 3)
-                    siddonForwardKernel<3><<<blocks, forwardThreads_, 0, s>>>(
-                        rays_->as<SiddonRay>(), nrays, x, vol_, binary_, y);
-                else
-                    siddonForwardKernel<2><<<blocks, forwardThreads_, 0, s>>>(
-                        rays_->as<SiddonRay>(), nrays, x, vol_, binary_, y);
+                SiddonLayouts layouts;
+                const int64_t plane = static_cast<int64_t>(vol_.n[0]) * vol_.n[1];
+                for (int g = 0; g < 3; ++g) {
+                    layouts.base[g] = x;
+                    layouts.stride[g][0] = 1, layouts.stride[g][1] = vol_.n[0];
+                    layouts.stride[g][2] = plane;
+                }
+                for (int f = 1; f < vol_.dim; ++f) {
+                    if (!copies_[f])
+                        continue;
+                    // axis f contiguous, then x, then the third axis
+                    const int64_t nf = vol_.n[f];
+                    int64_t stride[3];
+                    stride[f] = 1, stride[0] = nf, stride[3 - f] = nf * vol_.n[0];
+                    launchLayoutCopy(x, vol_, f, stride, copies_[f]->as<float>(), s);
+                    for (int g = 0; g < vol_.dim; ++g)
+                        if (fast_[g] == f) {
+                            layouts.base[g] = copies_[f]->as<float>();
+                            std::copy(stride, stride + 3, layouts.stride[g]);
+                        }
+                }
+                const bool narrow = domainSize_ < (int64_t(1) << 32);
+                auto* k = vol_.dim == 3 ? (narrow ? siddonForwardKernel<3, unsigned>
+                                                  : siddonForwardKernel<3, int64_t>)
+                                        : (narrow ? siddonForwardKernel<2, unsigned>
+                                                  : siddonForwardKernel<2, int64_t>);
+                k<<<blocks, forwardThreads_, 0, s>>>(rays_->as<SiddonRay>(), nrays, layouts, vol_,
+                                                     binary_, y);
                 ELSA_LAUNCH_CHECK("siddonForwardKernel");
             }
 
@@ -997,8 +1087,8 @@ namespace elsa_b200
                     return visits_;
                 case 3:
                     return 0;
-                case 6: // kernel launches per forward call
-                    return 1;
+                case 6: // kernel launches per forward call: the layout copies and the rays
+                    return 1 + (copies_[1] ? 1 : 0) + (copies_[2] ? 1 : 0);
                 case 7: // kernel launches per adjoint call (brick owner in 3D: one per axis
                         // grid; with several partial volumes: + the chunk sum)
                     if (scatter_)
@@ -1293,6 +1383,8 @@ namespace elsa_b200
             int binary_ = 0;
             CurvedDetector curved_;
             std::unique_ptr<DeviceBuffer> rays_, cpState_, cpVoxel_, viewAxes_, windows_;
+            std::array<int, 3> fast_{{0, 0, 0}};     // contiguous axis per driving axis (forward)
+            std::unique_ptr<DeviceBuffer> copies_[3]; // volume copies with axis 1 or 2 contiguous
             int cpRows_ = 0;
             int classSpacing_ = 0;
             int64_t visits_ = 0;

@@ -64,6 +64,21 @@ def test_joseph_2d_non_finite(cuda, oracle):
     assert np.array_equal(np.isinf(got), np.isinf(ref))
 
 
+@pytest.mark.parametrize("kind", ["SIDDON", "BINARY"])
+@pytest.mark.parametrize("vol,views,det", [
+    ((1, 1, 1), 3, [3, 3]), ((33, 31, 35), 7, [40, 33]), ((64, 5, 32), 8, [70, 9]),
+    ((1, 34, 67), 5, [90, 50]), ((33, 65), 9, [80]), ((1, 40), 6, [60])])
+def test_siddon_forward_layouts(cuda, oracle, vol, views, det, kind):
+    """Rays read from the volume or from a copy with another axis contiguous: the same visits and
+    sums, bit for bit."""
+    import elsa_b200
+    poses, det, x, _ = _problem(oracle, vol, views, det)
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    fn = oracle.siddon if kind == "SIDDON" else oracle.binary
+    ref = np.asarray(fn(x, vol, det, poses), np.float32)
+    assert np.array_equal(_apply(cuda, proj, x, False), ref)
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("kind,params", [
     ("blob", (2.0, 10.83, 2)), ("blob", (0.55, 10.83, 2)), ("blob", (3.7, 8.0, 1)),
