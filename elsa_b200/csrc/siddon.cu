@@ -102,6 +102,14 @@ namespace elsa_b200
             }
         }
 
+        __device__ __forceinline__ void crossIf(float tm, float& T, float tDelta, int& c, int step)
+        {
+            asm("{\n\t.reg .pred m;\n\tsetp.eq.f32 m, %0, %2;\n\t"
+                "@m add.rn.f32 %0, %0, %3;\n\t@m add.s32 %1, %1, %4;\n\t}"
+                : "+f"(T), "+r"(c)
+                : "f"(tm), "f"(tDelta), "r"(step));
+        }
+
         // Entry voxel in axis order from the record (g and the two other axes a < b).
         __device__ __forceinline__ void entryVoxel(int g, int kg, int ca, int cb, int& c0,
                                                    int& c1, int& c2)
@@ -675,63 +683,45 @@ namespace elsa_b200
             nonDrivingAxes(G, a, b);
             const int dirG = ((meta >> (2 + G)) & 1) ? -1 : 1;
             const int kg = dirG > 0 ? max(kLo, kFirst) : min(kLo + kSlab - 1, kFirst);
-            int c0, c1, c2;
-            entryVoxel(G, kg, static_cast<int>(cpv & 0xffffu), static_cast<int>(cpv >> 16), c0,
-                       c1, c2);
+            int c[3]; // voxel from the brick's first voxel
+            entryVoxel(G, kg, static_cast<int>(cpv & 0xffffu), static_cast<int>(cpv >> 16), c[0],
+                       c[1], c[2]);
+            c[G] -= kLo, c[a] -= orgA, c[b] -= orgB;
             const int s0 = axisStep(meta, 0), s1 = axisStep(meta, 1), s2 = axisStep(meta, 2);
             float T0 = cp.x, T1 = cp.y, T2 = cp.z;
             float tEntry = cp.w;
             // the walk stays inside the volume and the slab: along G the two tests are one,
             // kLo <= cg < min(kLo + kSlab, n_G)
-            const int nA = a == 0 ? vol.n[0] : (a == 1 ? vol.n[1] : vol.n[2]);
-            const int nB = b == 1 ? vol.n[1] : vol.n[2];
+            const unsigned nA = static_cast<unsigned>(a == 0 ? vol.n[0] : (a == 1 ? vol.n[1] : vol.n[2]));
+            const unsigned nB = static_cast<unsigned>(b == 1 ? vol.n[1] : vol.n[2]);
             const int nG = G == 0 ? vol.n[0] : (G == 1 ? vol.n[1] : vol.n[2]);
             const unsigned spanG = static_cast<unsigned>(min(kLo + kSlab, nG) - kLo);
+            const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(acc));
             // software-pipelined: the word of a visit is read before the sum of the previous
             // visit (always another voxel) is written back
-            int prevOff = 0;
+            unsigned prevAt = 0, prevIn = 0;
             float prevVal = 0.0f, prevW = 0.0f;
-            bool prevIn = false;
             for (int it = 0; it < 3 * kSlab + 3; ++it) {
-                bool m0, m1, m2;
-                const float tExit = nextCrossing<3>(T0, T1, T2, m0, m1, m2);
-                const int c[3] = {c0, c1, c2};
-                const int lg = c[G] - kLo, la = c[a] - orgA, lb = c[b] - orgB;
-                const bool in = static_cast<unsigned>(la) < static_cast<unsigned>(EA) &&
-                                static_cast<unsigned>(lb) < static_cast<unsigned>(EB);
-                const int off = lg * L::kPlane + la * SA + lb * SB;
-#if ELSA_SIDDON_NOZERO
-                float val; // read only where used: its store carries the same flag
-                if (in)
-                    val = acc[off];
-#else
-                const float val = in ? acc[off] : 0.0f;
-#endif
-                if (prevIn)
-                    acc[prevOff] = __fadd_rn(prevVal, __fmul_rn(yv, prevW));
-                prevOff = off, prevVal = val, prevIn = in;
+                const float tExit = fminf(T0, fminf(T1, T2));
+                const unsigned in = (static_cast<unsigned>(c[a]) < static_cast<unsigned>(EA)) &
+                                    (static_cast<unsigned>(c[b]) < static_cast<unsigned>(EB));
+                const unsigned at =
+                    base + 4u * static_cast<unsigned>(c[G] * L::kPlane + c[a] * SA + c[b] * SB);
+                float val;
+                loadSharedIf(val, at, in);
+                storeSharedIf(__fadd_rn(prevVal, __fmul_rn(yv, prevW)), prevAt, prevIn);
+                prevAt = at, prevVal = val, prevIn = in;
                 prevW = binary ? 1.0f : __fsub_rn(tExit, tEntry);
-                if (m0) {
-                    c0 += s0;
-                    T0 = __fadd_rn(T0, tDelta.x);
-                }
-                if (m1) {
-                    c1 += s1;
-                    T1 = __fadd_rn(T1, tDelta.y);
-                }
-                if (m2) {
-                    c2 += s2;
-                    T2 = __fadd_rn(T2, tDelta.z);
-                }
-                const int cn[3] = {c0, c1, c2};
-                if (static_cast<unsigned>(cn[a]) >= static_cast<unsigned>(nA) ||
-                    static_cast<unsigned>(cn[b]) >= static_cast<unsigned>(nB) ||
-                    static_cast<unsigned>(cn[G] - kLo) >= spanG)
+                crossIf(tExit, T0, tDelta.x, c[0], s0);
+                crossIf(tExit, T1, tDelta.y, c[1], s1);
+                crossIf(tExit, T2, tDelta.z, c[2], s2);
+                if ((static_cast<unsigned>(c[a] + orgA) >= nA) |
+                    (static_cast<unsigned>(c[b] + orgB) >= nB) |
+                    (static_cast<unsigned>(c[G]) >= spanG))
                     break;
                 tEntry = tExit;
             }
-            if (prevIn)
-                acc[prevOff] = __fadd_rn(prevVal, __fmul_rn(yv, prevW));
+            storeSharedIf(__fadd_rn(prevVal, __fmul_rn(yv, prevW)), prevAt, prevIn);
         }
 
         template <int G, bool UB>
