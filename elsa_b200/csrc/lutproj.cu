@@ -7,6 +7,7 @@
 // fixed-point atomic sums, so that the result is deterministic. As in the reference, the
 // adjoint walks the volume box grown by the support and the forward the volume box itself, so
 // the two are not exact transposes of each other near the box faces.
+#include "joseph_tma.cuh"
 #include "luts.hpp"
 #include "projector.hpp"
 #include "raysetup.cuh"
@@ -15,6 +16,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <memory>
 
 namespace elsa_b200
 {
@@ -79,20 +82,42 @@ namespace elsa_b200
                     mx = std::max(mx, std::fabs(v));
                 lp_.maxLut = mx;
                 traversalRotations(vol.dim, lp_.rot);
+                // rays that lead along x read a copy in which their rows' axis is contiguous
+                fast_ = 1;
+                if (vol.dim == 3) {
+                    std::vector<float> hp(poses_.size() * kPoseFloats);
+                    std::memcpy(hp.data(), poses_.data(), sizeof(float) * hp.size());
+                    fast_ = fastAxes(hp, det_)[0];
+                }
+                stride_[fast_] = 1, stride_[0] = vol.n[fast_];
+                stride_[3 - fast_] = static_cast<int64_t>(vol.n[fast_]) * vol.n[0];
+                try {
+                    copy_ = std::make_unique<DeviceBuffer>(sizeof(float) *
+                                                           static_cast<size_t>(domainSize_));
+                    second_ = std::make_unique<DeviceBuffer>(sizeof(unsigned long long) *
+                                                             static_cast<size_t>(domainSize_));
+                } catch (const Error&) { // no room: the x-fastest volume serves all rays
+                    cudaGetLastError();
+                }
                 ELSA_CUDA(cudaMemcpy(lut_.as<float>(), lut.values.data(),
                                      sizeof(float) * lut.values.size(), cudaMemcpyHostToDevice));
             }
 
             void forward(const float* x, float* y, cudaStream_t s) override
             {
-                launchLutForward(dPoses_, det_, lp_, lut_.as<float>(), x, y, s);
+                if (copy_)
+                    launchLayoutCopy(x, vol_, fast_, stride_, copy_->as<float>(), s);
+                launchLutForward(dPoses_, det_, lp_, lut_.as<float>(),
+                                 layouts(x, copy_ ? copy_->as<float>() : nullptr), y, s);
                 ELSA_LAUNCH_CHECK("lutForwardKernel");
             }
 
             void adjoint(const float* y, float* x, cudaStream_t s) override
             {
+                auto* acc = acc_.as<unsigned long long>();
+                auto* second = second_ ? second_->as<unsigned long long>() : nullptr;
                 launchLutBackward(dPoses_, det_, lp_, lut_.as<float>(), y, absMax_.as<unsigned>(),
-                                  acc_.as<unsigned long long>(), domainSize_, x, s);
+                                  acc, second, layouts(acc, second), stride_, domainSize_, x, s);
                 ELSA_LAUNCH_CHECK("lutBackwardKernel");
             }
 
@@ -100,7 +125,7 @@ namespace elsa_b200
             {
                 switch (key) {
                 case 6: // kernel launches per forward call
-                    return 1;
+                    return copy_ ? 2 : 1;
                 case 7: // per adjoint call: |y| maximum, fixed-point sums, conversion
                     return 3;
                 default:
@@ -109,6 +134,24 @@ namespace elsa_b200
             }
 
         private:
+            LutLayouts layouts(const void* base, const void* other) const
+            {
+                LutLayouts l;
+                for (int g = 0; g < 3; ++g) {
+                    l.base[g] = base;
+                    l.stride[g][0] = 1, l.stride[g][1] = vol_.n[0];
+                    l.stride[g][2] = static_cast<int64_t>(vol_.n[0]) * vol_.n[1];
+                }
+                if (other) {
+                    l.base[0] = other;
+                    std::copy(stride_, stride_ + 3, l.stride[0]);
+                }
+                return l;
+            }
+
+            int fast_ = 1;        // contiguous axis of the copy for rays that lead along x
+            int64_t stride_[3];   // its strides
+            std::unique_ptr<DeviceBuffer> copy_, second_; // volume copy, second set of sums
             DeviceBuffer lut_, absMax_, acc_;
             LutProjParams lp_{};
         };

@@ -38,6 +38,7 @@ namespace elsa_b200
         int support;
         float radius;
         float maxLut;
+        float minusZero = -0.0f; // see lutRayAlong
         float rot[6][9];
     };
 
@@ -54,10 +55,23 @@ namespace elsa_b200
         return ldexp(1.0, 62 - e);
     }
 
+    // Per leading axis of a ray, the copy of the volume (or of the sums) it works on: the x-fastest
+    // one, or one in which the axis is contiguous along which neighbouring rays spread (a warp
+    // whose rays lead along x otherwise touches 32 sectors per voxel); strides in words.
+    struct LutLayouts {
+        const void* base[3];
+        int64_t stride[3][3];
+    };
+
+    // layouts: float copies of the volume
     void launchLutForward(const float* poses, const DetectorShape& det, const LutProjParams& lp,
-                          const float* lut, const float* x, float* y, cudaStream_t s);
-    // absMaxBits: one device word of scratch; acc: nvox 64-bit words of scratch
+                          const float* lut, const LutLayouts& layouts, float* y, cudaStream_t s);
+    // absMaxBits: one device word of scratch; acc: nvox 64-bit words of scratch (x fastest);
+    // second: null or another nvox words with strides secondStride; layouts: which of the two the
+    // rays of a leading axis add to
     void launchLutBackward(const float* poses, const DetectorShape& det, const LutProjParams& lp,
                            const float* lut, const float* y, unsigned* absMaxBits,
-                           unsigned long long* acc, int64_t nvox, float* x, cudaStream_t s);
+                           unsigned long long* acc, unsigned long long* second,
+                           const LutLayouts& layouts, const int64_t (&secondStride)[3],
+                           int64_t nvox, float* x, cudaStream_t s);
 } // namespace elsa_b200
