@@ -188,9 +188,8 @@ namespace elsa_b200
         t.mark(s);
         A.adjoint(sino, q, s); // q = A^T A c
         t.mark(s);
-        launchDot(c, q, n, partials, &S->den, s);    // <c, A^T A c>
-        launchCgStep(x, r, c, q, n, S, partials, s); // x += a c, r -= a q, |r|^2 partials
-        launchCgFinishNorm(partials, S, s);          // k, beta = k/kold, kold = k
+        launchCgDen(c, q, n, S, partials, s);        // <c, A^T A c>
+        launchCgStep(x, r, c, q, n, S, partials, s); // x += a c, r -= a q; beta = k/kold, kold = k
         launchCgDirection(r, c, n, S, s);            // c = r + beta c
     }
 
@@ -231,9 +230,8 @@ namespace elsa_b200
         float* c = ws_.vol1.as<float>();
         double* partials = ws_.partials.as<double>();
         SolverScalars* S = ws_.scalars.as<SolverScalars>();
-        launchDot(c, q, n, partials, &S->den, s);     // <c, sum_r A_r^T A_r c>
-        launchCgStep(x_, r, c, q, n, S, partials, s); // x += a c, r -= a q, |r|^2 partials
-        launchCgFinishNorm(partials, S, s);           // k, beta = k/kold, kold = k
+        launchCgDen(c, q, n, S, partials, s);         // <c, sum_r A_r^T A_r c>
+        launchCgStep(x_, r, c, q, n, S, partials, s); // x += a c, r -= a q; beta, kold = |r|^2
         launchCgDirection(r, c, n, S, s);             // c = r + beta c
     }
 

@@ -171,7 +171,7 @@ namespace elsa_b200
 
     // Many CGNE solves (x0 = 0) on 3D Joseph operators advanced together: per iteration every
     // operator's forward (fanned out over side streams), then all matched adjoints in one launch
-    // per driving-axis grid (planJosephAdjointMany), then all vector updates in five launches
+    // per driving-axis grid (planJosephAdjointMany), then all vector updates in three launches
     // (launchCgneUpdateBatch). Every instance's iterates equal those of its own SolverSession
     // bit for bit. iterateGraph captures the batched iterations as one CUDA graph.
     class BatchedCgne

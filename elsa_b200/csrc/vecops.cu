@@ -76,12 +76,48 @@ namespace elsa_b200
                 partials[blockIdx.x] = s;
         }
 
-        __device__ __forceinline__ double sumPartials(const double* __restrict__ partials)
+        __device__ __forceinline__ double sumPartials(const double* partials)
         {
             double v = 0.0;
             for (int i = threadIdx.x; i < kReduceBlocks; i += blockDim.x)
-                v += partials[i];
+                v += __ldcg(partials + i); // (written by the same launch in lastBlock's callers)
             return blockSum(v);
+        }
+
+        // Whether this block is the last of a kReduceBlocks-wide reduction to get here, its
+        // partial sum written by thread 0: that block then adds the partials, in block order, in
+        // place of a launch of its own (at 128^2 a CGNE iteration has 3 vector launches instead of
+        // 5). The ticket is back at 0 afterwards.
+        __device__ __forceinline__ bool lastBlock(unsigned* ticket)
+        {
+            __shared__ bool last;
+            if (threadIdx.x == 0) {
+                __threadfence();
+                last = atomicInc(ticket, kReduceBlocks - 1) == kReduceBlocks - 1;
+                __threadfence();
+            }
+            __syncthreads();
+            return last;
+        }
+
+        // <c, q> into S->den by the last block.
+        __device__ __forceinline__ void cgDen(const float* __restrict__ c,
+                                              const float* __restrict__ q, int64_t n,
+                                              SolverScalars* S, double* partials)
+        {
+            partialDot<false>(c, q, n, partials);
+            if (!lastBlock(&S->ticket))
+                return;
+            const double s = sumPartials(partials);
+            if (threadIdx.x == 0)
+                S->den = s;
+        }
+
+        __global__ void __launch_bounds__(kReduceThreads)
+            cgDenKernel(const float* __restrict__ c, const float* __restrict__ q, int64_t n,
+                        SolverScalars* S, double* partials)
+        {
+            cgDen(c, q, n, S, partials);
         }
 
         __global__ void __launch_bounds__(kReduceThreads)
@@ -132,13 +168,12 @@ namespace elsa_b200
         __device__ __forceinline__ void cgStep(float* __restrict__ x, float* __restrict__ r,
                                                const float* __restrict__ c,
                                                const float* __restrict__ q, int64_t n,
-                                               const SolverScalars* S,
-                                               double* __restrict__ partials);
+                                               SolverScalars* S, double* partials);
 
         __global__ void __launch_bounds__(kReduceThreads)
             cgStepKernel(float* __restrict__ x, float* __restrict__ r, const float* __restrict__ c,
-                         const float* __restrict__ q, int64_t n, const SolverScalars* S,
-                         double* __restrict__ partials)
+                         const float* __restrict__ q, int64_t n, SolverScalars* S,
+                         double* partials)
         {
             cgStep(x, r, c, q, n, S, partials);
         }
@@ -146,8 +181,7 @@ namespace elsa_b200
         __device__ __forceinline__ void cgStep(float* __restrict__ x, float* __restrict__ r,
                                                const float* __restrict__ c,
                                                const float* __restrict__ q, int64_t n,
-                                               const SolverScalars* S,
-                                               double* __restrict__ partials)
+                                               SolverScalars* S, double* partials)
         {
             const float alpha = static_cast<float>(S->kold / S->den);
             const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -159,9 +193,18 @@ namespace elsa_b200
                 r[i] = ri;
                 acc += static_cast<double>(ri) * ri;
             }
-            const double s = blockSum(acc);
+            double s = blockSum(acc);
             if (threadIdx.x == 0)
                 partials[blockIdx.x] = s;
+            // every block has read the scalars before the last one gets here
+            if (!lastBlock(&S->ticket))
+                return;
+            s = sumPartials(partials);
+            if (threadIdx.x == 0) {
+                S->k = s;
+                S->beta = s / S->kold;
+                S->kold = s;
+            }
         }
 
         __global__ void __launch_bounds__(kReduceThreads)
@@ -173,14 +216,6 @@ namespace elsa_b200
                 S->beta = s / S->kold;
                 S->kold = s;
             }
-        }
-
-        __global__ void __launch_bounds__(kReduceThreads)
-            finishDenKernel(const double* __restrict__ partials, SolverScalars* S)
-        {
-            const double s = sumPartials(partials);
-            if (threadIdx.x == 0)
-                S->den = s;
         }
 
         __global__ void cgDirectionKernel(const float* __restrict__ r, float* __restrict__ c,
@@ -199,16 +234,7 @@ namespace elsa_b200
             dotManyKernel(const CgBatchEntry* __restrict__ e)
         {
             const CgBatchEntry E = e[blockIdx.y];
-            partialDot<false>(E.c, E.q, E.n, E.partials);
-        }
-
-        __global__ void __launch_bounds__(kReduceThreads)
-            finishDenManyKernel(const CgBatchEntry* __restrict__ e)
-        {
-            const CgBatchEntry E = e[blockIdx.y];
-            const double s = sumPartials(E.partials);
-            if (threadIdx.x == 0)
-                E.S->den = s;
+            cgDen(E.c, E.q, E.n, E.S, E.partials);
         }
 
         __global__ void __launch_bounds__(kReduceThreads)
@@ -216,18 +242,6 @@ namespace elsa_b200
         {
             const CgBatchEntry E = e[blockIdx.y];
             cgStep(E.x, E.r, E.c, E.q, E.n, E.S, E.partials);
-        }
-
-        __global__ void __launch_bounds__(kReduceThreads)
-            cgFinishNormManyKernel(const CgBatchEntry* __restrict__ e)
-        {
-            const CgBatchEntry E = e[blockIdx.y];
-            const double s = sumPartials(E.partials);
-            if (threadIdx.x == 0) {
-                E.S->k = s;
-                E.S->beta = s / E.S->kold;
-                E.S->kold = s;
-            }
         }
 
         __global__ void cgDirectionManyKernel(const CgBatchEntry* __restrict__ e)
@@ -289,6 +303,13 @@ namespace elsa_b200
         ELSA_LAUNCH_CHECK("scale");
     }
 
+    void launchCgDen(const float* c, const float* q, int64_t n, SolverScalars* S, double* partials,
+                     cudaStream_t s)
+    {
+        cgDenKernel<<<kReduceBlocks, kReduceThreads, 0, s>>>(c, q, n, S, partials);
+        ELSA_LAUNCH_CHECK("cgDen");
+    }
+
     void launchCgStep(float* x, float* r, const float* c, const float* q, int64_t n,
                       SolverScalars* S, double* partials, cudaStream_t s)
     {
@@ -300,12 +321,6 @@ namespace elsa_b200
     {
         cgFinishNormKernel<<<1, kReduceThreads, 0, s>>>(partials, S);
         ELSA_LAUNCH_CHECK("cgFinishNorm");
-    }
-
-    void launchFinishDen(const double* partials, SolverScalars* S, cudaStream_t s)
-    {
-        finishDenKernel<<<1, kReduceThreads, 0, s>>>(partials, S);
-        ELSA_LAUNCH_CHECK("finishDen");
     }
 
     void launchCgDirection(const float* r, float* c, int64_t n, const SolverScalars* S,
@@ -322,9 +337,7 @@ namespace elsa_b200
             return;
         const unsigned nb = static_cast<unsigned>(count);
         dotManyKernel<<<dim3(kReduceBlocks, nb), kReduceThreads, 0, s>>>(entries);
-        finishDenManyKernel<<<dim3(1, nb), kReduceThreads, 0, s>>>(entries);
         cgStepManyKernel<<<dim3(kReduceBlocks, nb), kReduceThreads, 0, s>>>(entries);
-        cgFinishNormManyKernel<<<dim3(1, nb), kReduceThreads, 0, s>>>(entries);
         cgDirectionManyKernel<<<dim3(gridFor(maxN), nb), 256, 0, s>>>(entries);
         ELSA_LAUNCH_CHECK("cgneUpdateBatch");
     }

@@ -25,7 +25,7 @@ namespace elsa_b200
         double tPrev;  // FISTA momentum t_{k-1}
         double aux[2]; // aux[0]: |c|^2 for damped CGLS
         int done;      // set once a convergence test passed; later updates become no-ops
-        int pad;
+        unsigned ticket; // blocks of the running reduction that are done (0 between launches)
     };
 
     // Proximal operators of APGD (proximal_operators/ProximalBoxConstraint.cpp,
@@ -51,7 +51,7 @@ namespace elsa_b200
 
     // The CGNE update (dot <c, q> -> den, step, norm, direction) of `count` instances in five
     // launches; every instance runs the blocks and summation order of the single-instance
-    // launches (launchDot, launchCgStep, launchCgFinishNorm, launchCgDirection), so its results
+    // launches (launchCgDen, launchCgStep, launchCgDirection), so its results
     // are bit-identical to theirs. entries: device array; maxN: largest n.
     void launchCgneUpdateBatch(const CgBatchEntry* entries, int count, int64_t maxN,
                                cudaStream_t s);
@@ -71,13 +71,15 @@ namespace elsa_b200
     void launchScale(float* x, float value, int64_t n, cudaStream_t s);
 
     // CG building blocks (see CGNE/CGLS in solvers.cu).
-    // x += alpha*c; r -= alpha*q with alpha = S->kold / S->den; partial sums of |r|^2.
+    // S->den = <c, q>
+    void launchCgDen(const float* c, const float* q, int64_t n, SolverScalars* S, double* partials,
+                     cudaStream_t s);
+    // x += alpha*c; r -= alpha*q with alpha = S->kold / S->den; then S->k = |r|^2,
+    // S->beta = S->k / S->kold, S->kold = S->k
     void launchCgStep(float* x, float* r, const float* c, const float* q, int64_t n,
                       SolverScalars* S, double* partials, cudaStream_t s);
     // S->k = sum(partials); S->beta = S->k / S->kold; S->kold = S->k
     void launchCgFinishNorm(const double* partials, SolverScalars* S, cudaStream_t s);
-    // S->den = sum(partials) (+ extra * S->aux[0] if extra != 0)
-    void launchFinishDen(const double* partials, SolverScalars* S, cudaStream_t s);
     // c = r + beta*c
     void launchCgDirection(const float* r, float* c, int64_t n, const SolverScalars* S,
                            cudaStream_t s);

@@ -390,7 +390,7 @@ typedef enum elsa_solver_kind {
  * solves A_i^T A_i x_i = A_i^T b_i from x_i = 0 with its own operator (a 3D Joseph projector
  * with the matched adjoint; others return ELSA_ERROR_NOT_SUPPORTED), b_i and x_i device
  * buffers. Per iteration the instances' forwards run concurrently, all adjoints run in one
- * launch per driving-axis grid over an instance table, and all vector updates in five launches;
+ * launch per driving-axis grid over an instance table, and all vector updates in three launches;
  * every x_i equals what a single elsa_solver session computes, bit for bit.
  * elsa_batch_cgne_iterate_graph captures the batched iterations as one CUDA graph (stream must
  * be an explicitly created stream). residuals: count doubles |r_i|^2 in host memory
