@@ -36,49 +36,6 @@ namespace elsa_b200
         constexpr int kStageFloats = BW * BH * BD;
         constexpr unsigned kStageBytes = kStageFloats * sizeof(float);
         constexpr int kFlagFallback = 8;
-#ifndef ELSA_FWD_FULLCHUNK
-#define ELSA_FWD_FULLCHUNK 1 // warp-uniform fast path for chunks without partial rays
-#endif
-#ifndef ELSA_FWD_NOCLAMP
-#define ELSA_FWD_NOCLAMP 1 // taps indexed without clamps (in range by construction)
-#endif
-
-#ifndef ELSA_FWD_PAIR_ACC
-#define ELSA_FWD_PAIR_ACC 1 // the two footprint rows summed separately, one packed fma per sample
-                            // (256^3: 10.61 -> 10.49 ms)
-#endif
-#ifndef ELSA_FWD_PACKED
-#define ELSA_FWD_PACKED 1 // the (fast, slow) pairs on the packed two-wide FP32 instructions
-                          // (256^3: 12.04 -> 10.59 ms)
-#endif
-#ifndef ELSA_FWD_MAGIC_FLOOR
-#define ELSA_FWD_MAGIC_FLOOR 1
-#endif
-        // floor of a tap coordinate and its integer: floorSmall on the FMA and integer pipes
-        // (the conversion pipe is 62 % busy in this kernel otherwise; 256^3: 12.27 -> 12.04 ms),
-        // or floorf and a conversion with ELSA_FWD_MAGIC_FLOOR 0; the same values.
-        [[maybe_unused]] __device__ __forceinline__ float floorTap(float x, int& i)
-        {
-#if ELSA_FWD_MAGIC_FLOOR
-            return floorSmall(x, i);
-#else
-            const float f = floorf(x);
-            i = static_cast<int>(f);
-            return f;
-#endif
-        }
-
-        // Tap index along a box edge of E words. The box origins of every (tile, chunk) come from
-        // the same accumulated positions (tileSetupKernel: identical float operations, and a tile
-        // whose samples do not fit its boxes takes the per-ray gather), so i is in [0, E - 2] by
-        // construction and needs no clamp; ELSA_FWD_NOCLAMP 0 clamps it anyway.
-        // 256^3 / 360 views: 14.55 ms clamped, 13.84 ms without; 12.27 ms with the full-chunk
-        // fast path as well.
-        template <int E>
-        __device__ __forceinline__ int boxIndex(int i)
-        {
-            return ELSA_FWD_NOCLAMP ? i : min(max(i, 0), E - 2);
-        }
 
         __device__ __forceinline__ int floorDivI(int a, int b)
         {
@@ -340,6 +297,67 @@ namespace elsa_b200
             return R.len * acc;
         }
 
+        // v = the shared word at byte address p where cond != 0, else v as it is (ordered with the
+        // barrier waits, as every volatile asm).
+        __device__ __forceinline__ void readSharedIf(float& v, unsigned p, unsigned cond)
+        {
+            asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %2, 0;\n\t"
+                         "@t ld.shared.f32 %0, [%1];\n\t}"
+                         : "+f"(v)
+                         : "r"(p), "r"(cond));
+        }
+
+        // Samples of one chunk of a ray: p2 the (fast, slow) position of its next sample, acc the
+        // sums of the two footprint rows (their interpolation along fast; the one along slow is
+        // the weights w.y and cw.y). DIR: the ray's direction, so that a sample's plane is an
+        // immediate offset. Full: all BD samples; otherwise those with 0 <= jBase + kk < n.
+        // origin: word of the chunk's stage buffer less the box origin and the bias of the two
+        // floors' bit patterns (floorSmall2). The box origins of every (tile, chunk) come from the
+        // same accumulated positions (tileSetupKernel: identical float operations, and a tile
+        // whose samples do not fit its boxes takes the per-ray gather), so every tap lies in its
+        // box and no index is clamped.
+        // Bound by issue: about 20 instructions per sample (position, floors and weights packed
+        // two-wide). 256^3 / 360 views / 384^2: 10.41 -> 9.40 ms.
+        template <int DIR, bool Full>
+        __device__ __forceinline__ void chunkSamples(const float* stage, unsigned origin,
+                                                     float2& p2, float2 s2, float2& acc, int jBase,
+                                                     int n)
+        {
+            const float2 magic = make_float2(12582912.0f, 12582912.0f); // 1.5 * 2^23
+            const float2 half = make_float2(0.5f, 0.5f), one = make_float2(1.0f, 1.0f);
+#pragma unroll
+            for (int kk = 0; kk < BD; ++kk) {
+                const float2 h = sub2(p2, half);
+                const float2 t = add2Down(h, magic);
+                const float2 cw = sub2(h, sub2(t, magic));
+                const float2 w = sub2(one, cw);
+                const int word = static_cast<int>(__float_as_uint(t.y) * BW +
+                                                  __float_as_uint(t.x) + origin);
+                const int plane = (DIR > 0 ? kk : BD - 1 - kk) * (BW * BH);
+                if (Full) {
+                    const float* q = stage + word + plane;
+                    acc.x = __fmaf_rn(w.y, __fmaf_rn(cw.x, q[1], w.x * q[0]), acc.x);
+                    acc.y = __fmaf_rn(cw.y, __fmaf_rn(cw.x, q[BW + 1], w.x * q[BW]), acc.y);
+                    p2 = add2(p2, s2);
+                } else {
+                    // predicated, not branched around: half of the warps would diverge
+                    const unsigned on = static_cast<unsigned>(jBase + kk) <
+                                        static_cast<unsigned>(n);
+                    const unsigned q = static_cast<unsigned>(__cvta_generic_to_shared(stage)) +
+                                       4u * static_cast<unsigned>(word + plane);
+                    float v00 = 0.0f, v10 = 0.0f, v01 = 0.0f, v11 = 0.0f;
+                    readSharedIf(v00, q, on);
+                    readSharedIf(v10, q + 4, on);
+                    readSharedIf(v01, q + 4 * BW, on);
+                    readSharedIf(v11, q + 4 * BW + 4, on);
+                    acc.x = __fmaf_rn(w.y, __fmaf_rn(cw.x, v10, w.x * v00), acc.x);
+                    acc.y = __fmaf_rn(cw.y, __fmaf_rn(cw.x, v11, w.x * v01), acc.y);
+                    const float2 next = add2(p2, s2);
+                    p2 = on ? next : p2;
+                }
+            }
+        }
+
         __global__ void __launch_bounds__(NT)
             forwardTmaKernel(const __grid_constant__ CUtensorMap map0,
                              const __grid_constant__ CUtensorMap map1,
@@ -403,17 +421,11 @@ namespace elsa_b200
             if (threadIdx.x == 0)
                 for (int ch = 0; ch < NS && ch < T.nChunks; ++ch)
                     issue(ch);
-            float acc = 0.0f;
-#if ELSA_FWD_PACKED
-#if ELSA_FWD_PAIR_ACC
-            float2 acc2 = make_float2(0.0f, 0.0f); // the two footprint rows' sums
-#endif
-            float2 p2 = make_float2(c.pf, c.ps); // (fast, slow) position
+            float2 acc = make_float2(0.0f, 0.0f); // the two footprint rows' sums
+            float2 p2 = make_float2(c.pf, c.ps);  // (fast, slow) position
             const float2 s2 = make_float2(c.sf, c.ss);
-#else
-            float pf = c.pf, ps = c.ps;
-#endif
             int failed = -1; // chunk whose wait timed out
+            int2 ahead = T.nChunks > 0 ? org[0] : make_int2(0, 0); // next chunk's box origin
             for (int ch = 0; ch < T.nChunks; ++ch) {
                 const int s = ch % NS;
                 const bool ready = mbarWait(&full[s], (ch / NS) & 1, waitCycles);
@@ -421,94 +433,26 @@ namespace elsa_b200
                     atomicOr(error, 1u);
                     abortFlag = 1;
                 }
-                const int2 o = org[ch];
-                const float* buf = stage + s * kStageFloats;
+                const int2 o = ahead;
+                if (ch + 1 < T.nChunks)
+                    ahead = org[ch + 1];
+                const unsigned origin = static_cast<unsigned>(s * kStageFloats) -
+                                        (0x4B400000u + static_cast<unsigned>(o.x)) -
+                                        (0x4B400000u + static_cast<unsigned>(o.y)) * BW;
                 const int jBase = ch * BD - c.t0;
-#if ELSA_FWD_FULLCHUNK
                 // chunks in which every ray of the warp has all BD samples: no per-sample test
-                if (__all_sync(0xffffffffu, ready && jBase >= 0 && jBase + BD <= c.n)) {
-#pragma unroll
-                    for (int kk = 0; kk < BD; ++kk) {
-#if ELSA_FWD_PACKED
-                        // (f, s) pairs on the packed two-wide FP32 path: the same roundings
-                        int fi, si;
-                        const float2 h = make_float2(0.5f, 0.5f);
-                        const float2 fl = floorSmall2(sub2(p2, h), fi, si);
-                        const float2 cw = sub2(sub2(p2, fl), h);
-                        const float2 w = sub2(make_float2(1.0f, 1.0f), cw);
-                        const int lf = boxIndex<BW>(fi - o.x);
-                        const int ls = boxIndex<BH>(si - o.y);
-                        const int lk = dir > 0 ? kk : BD - 1 - kk;
-                        const float* q = buf + (lk * BH + ls) * BW + lf;
-                        // rows v0 and v1 of the footprint: (wf v00 + cwf v10, wf v01 + cwf v11)
-                        const float2 r = fma2(make_float2(cw.x, cw.x), make_float2(q[1], q[BW + 1]),
-                                              mul2(make_float2(w.x, w.x), make_float2(q[0], q[BW])));
-#if ELSA_FWD_PAIR_ACC
-                        acc2 = fma2(make_float2(w.y, cw.y), r, acc2);
-#else
-                        acc += w.y * r.x + cw.y * r.y;
-#endif
-                        p2 = add2(p2, s2);
-#else
-                        int fi, si;
-                        const float ff = floorTap(__fsub_rn(pf, 0.5f), fi);
-                        const float fs = floorTap(__fsub_rn(ps, 0.5f), si);
-                        const float cwf = __fsub_rn(__fsub_rn(pf, ff), 0.5f);
-                        const float cws = __fsub_rn(__fsub_rn(ps, fs), 0.5f);
-                        const float wf = __fsub_rn(1.0f, cwf), ws = __fsub_rn(1.0f, cws);
-                        const int lf = boxIndex<BW>(fi - o.x);
-                        const int ls = boxIndex<BH>(si - o.y);
-                        const int lk = dir > 0 ? kk : BD - 1 - kk;
-                        const float* q = buf + (lk * BH + ls) * BW + lf;
-                        const float v00 = q[0], v10 = q[1], v01 = q[BW], v11 = q[BW + 1];
-                        acc += ws * (wf * v00 + cwf * v10) + cws * (wf * v01 + cwf * v11);
-                        pf = __fadd_rn(pf, c.sf);
-                        ps = __fadd_rn(ps, c.ss);
-#endif
-                    }
-                } else
-#endif
-#pragma unroll
-                for (int kk = 0; kk < BD; ++kk) {
-                    const int j = jBase + kk;
-                    if (ready && j >= 0 && j < c.n) {
-#if ELSA_FWD_PACKED
-                        // (f, s) pairs on the packed two-wide FP32 path: the same roundings
-                        int fi, si;
-                        const float2 h = make_float2(0.5f, 0.5f);
-                        const float2 fl = floorSmall2(sub2(p2, h), fi, si);
-                        const float2 cw = sub2(sub2(p2, fl), h);
-                        const float2 w = sub2(make_float2(1.0f, 1.0f), cw);
-                        const int lf = boxIndex<BW>(fi - o.x);
-                        const int ls = boxIndex<BH>(si - o.y);
-                        const int lk = dir > 0 ? kk : BD - 1 - kk;
-                        const float* q = buf + (lk * BH + ls) * BW + lf;
-                        // rows v0 and v1 of the footprint: (wf v00 + cwf v10, wf v01 + cwf v11)
-                        const float2 r = fma2(make_float2(cw.x, cw.x), make_float2(q[1], q[BW + 1]),
-                                              mul2(make_float2(w.x, w.x), make_float2(q[0], q[BW])));
-#if ELSA_FWD_PAIR_ACC
-                        acc2 = fma2(make_float2(w.y, cw.y), r, acc2);
-#else
-                        acc += w.y * r.x + cw.y * r.y;
-#endif
-                        p2 = add2(p2, s2);
-#else
-                        int fi, si;
-                        const float ff = floorTap(__fsub_rn(pf, 0.5f), fi);
-                        const float fs = floorTap(__fsub_rn(ps, 0.5f), si);
-                        const float cwf = __fsub_rn(__fsub_rn(pf, ff), 0.5f);
-                        const float cws = __fsub_rn(__fsub_rn(ps, fs), 0.5f);
-                        const float wf = __fsub_rn(1.0f, cwf), ws = __fsub_rn(1.0f, cws);
-                        const int lf = boxIndex<BW>(fi - o.x);
-                        const int ls = boxIndex<BH>(si - o.y);
-                        const int lk = dir > 0 ? kk : BD - 1 - kk;
-                        const float* q = buf + (lk * BH + ls) * BW + lf;
-                        const float v00 = q[0], v10 = q[1], v01 = q[BW], v11 = q[BW + 1];
-                        acc += ws * (wf * v00 + cwf * v10) + cws * (wf * v01 + cwf * v11);
-                        pf = __fadd_rn(pf, c.sf);
-                        ps = __fadd_rn(ps, c.ss);
-#endif
-                    }
+                const bool full = __all_sync(0xffffffffu, ready && jBase >= 0 && jBase + BD <= c.n);
+                const int n = ready ? c.n : 0;
+                if (dir > 0) {
+                    if (full)
+                        chunkSamples<1, true>(stage, origin, p2, s2, acc, jBase, n);
+                    else
+                        chunkSamples<1, false>(stage, origin, p2, s2, acc, jBase, n);
+                } else {
+                    if (full)
+                        chunkSamples<-1, true>(stage, origin, p2, s2, acc, jBase, n);
+                    else
+                        chunkSamples<-1, false>(stage, origin, p2, s2, acc, jBase, n);
                 }
                 __syncthreads();
                 if (abortFlag) { // a copy never completed: issue no more
@@ -526,11 +470,8 @@ namespace elsa_b200
                         mbarWait(&full[ch % NS], (ch / NS) & 1, waitCycles);
                 __syncthreads();
             }
-#if ELSA_FWD_PACKED && ELSA_FWD_PAIR_ACC
-            acc = acc2.x + acc2.y;
-#endif
             if (valid)
-                y[r] = c.n > 0 ? R.len * acc : 0.0f;
+                y[r] = c.n > 0 ? R.len * (acc.x + acc.y) : 0.0f;
         }
     } // namespace
 
