@@ -77,6 +77,11 @@ namespace elsa_b200
                 lp_.lutN = static_cast<int>(lut.values.size());
                 lp_.support = support;
                 lp_.radius = lut.support;
+                {
+                    int e = 0;
+                    if (std::frexp(lut.support, &e) == 0.5f)
+                        lp_.exactInv = std::ldexp(1.0f, 1 - e);
+                }
                 float mx = 0.0f;
                 for (float v : lut.values)
                     mx = std::max(mx, std::fabs(v));

@@ -38,6 +38,7 @@ namespace elsa_b200
         int support;
         float radius;
         float maxLut;
+        float exactInv = 0.0f;   // 1 / radius where the radius is a power of two, else 0
         float minusZero = -0.0f; // see lutRayAlong
         float rot[6][9];
     };
