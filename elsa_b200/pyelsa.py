@@ -176,9 +176,16 @@ class DataContainer:
 
     @classmethod
     def zeros(cls, descriptor):
+        obj = cls._empty(descriptor)
+        obj.tensor.zero_()
+        return obj
+
+    @classmethod
+    def _empty(cls, descriptor):
+        """For outputs that a native call overwrites whole."""
         torch = _torch()
         obj = cls.__new__(cls)
-        obj.tensor = torch.zeros(descriptor.getNumberOfCoefficients(), dtype=torch.float32,
+        obj.tensor = torch.empty(descriptor.getNumberOfCoefficients(), dtype=torch.float32,
                                  device="cuda")
         obj.descriptor = descriptor
         return obj
@@ -225,7 +232,7 @@ class DataContainer:
         """a * self + b * other (elsa_lincomb, core/DataContainer.cpp:1075-1108)."""
         import ctypes
         o = _as_dc(other, self.descriptor) if other is not None else self
-        out = DataContainer.zeros(self.descriptor)
+        out = DataContainer._empty(self.descriptor)
         _capi.call("elsa_lincomb", ctypes.c_float(a), ctypes.c_void_p(self._ptr()),
                    ctypes.c_float(b), ctypes.c_void_p(o._ptr()), ctypes.c_void_p(out._ptr()),
                    self.getSize(), ctypes.c_void_p(self._stream()))
@@ -292,13 +299,13 @@ class LinearOperator:
 
     def apply(self, x, Ax=None):
         x = _as_dc(x, self._domain)
-        out = Ax if Ax is not None else DataContainer.zeros(self._range)
+        out = Ax if Ax is not None else DataContainer._empty(self._range)
         self._op.apply_ptr(x._ptr(), _as_dc(out, self._range)._ptr(), self._stream())
         return out
 
     def applyAdjoint(self, y, Aty=None):
         y = _as_dc(y, self._range)
-        out = Aty if Aty is not None else DataContainer.zeros(self._domain)
+        out = Aty if Aty is not None else DataContainer._empty(self._domain)
         self._op.apply_adjoint_ptr(y._ptr(), _as_dc(out, self._domain)._ptr(), self._stream())
         return out
 
