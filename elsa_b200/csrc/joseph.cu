@@ -1316,12 +1316,10 @@ namespace elsa_b200
                 const int tile = domainSize_ <= kSmallImage ? 32 : 64;
                 brick_ = make_int3(tile, tile, 1);
                 buildCheckpoints(tile);
-                rows_ = std::make_unique<DeviceBuffer>(sizeof(float) * vol_.n[1] *
-                                                       linePitch(vol_.n[0]));
-                columns_ = std::make_unique<DeviceBuffer>(sizeof(float) * vol_.n[0] *
-                                                          linePitch(vol_.n[1]));
-                ELSA_CUDA(cudaMemset(rows_->as<float>(), 0, rows_->bytes()));
-                ELSA_CUDA(cudaMemset(columns_->as<float>(), 0, columns_->bytes()));
+                lines_ = std::make_unique<StreamScratch>(
+                    sizeof(float) * (rowWords() + static_cast<size_t>(vol_.n[0]) *
+                                                      linePitch(vol_.n[1])));
+                ELSA_CUDA(cudaMemset(lines_->initial(), 0, lines_->bytes()));
             }
 
             // Per view and driving axis g: set bit 4+g of the view's axis word when neighbouring
@@ -1455,11 +1453,21 @@ namespace elsa_b200
                     forward2d(x, y, s);
             }
 
+            size_t rowWords() const // words of the padded rows, a multiple of 4
+            {
+                return static_cast<size_t>(vol_.n[1]) * linePitch(vol_.n[0]);
+            }
+
             void forward2d(const float* x, float* y, cudaStream_t s)
             {
+                const StreamScratch::Lease lines(*lines_, s);
+                if (lines.own()) // the padding
+                    ELSA_CUDA(cudaMemsetAsync(lines.as<void>(), 0, lines_->bytes(), s));
+                float* rows = lines.as<float>();
+                float* columns = rows + rowWords();
                 const dim3 blocks((vol_.n[0] + 31) / 32, (vol_.n[1] + 31) / 32);
                 padLinesKernel<<<blocks, dim3(32, 8), 0, s>>>(
-                    x, vol_.n[0], vol_.n[1], rows_->as<float>(), columns_->as<float>());
+                    x, vol_.n[0], vol_.n[1], rows, columns);
                 ELSA_LAUNCH_CHECK("padLinesKernel");
                 const int depth = 1 << cpdShift_;
                 const int slabs = (std::max(vol_.n[0], vol_.n[1]) + depth - 1) / depth;
@@ -1475,8 +1483,7 @@ namespace elsa_b200
                     static_cast<int64_t>(segments) * ((det_.np + groups - 1) / groups);
                 josephForward2dKernel<<<static_cast<unsigned>(grid), dim3(32, groups * perGroup), 0,
                                         s>>>(dRays_, dCheckpoints_, rangeSize_, vol_, det_, depth,
-                                             slabs, groups, segments, rows_->as<float>(),
-                                             columns_->as<float>(), y);
+                                             slabs, groups, segments, rows, columns, y);
                 ELSA_LAUNCH_CHECK("josephForward2dKernel");
             }
 
@@ -1852,7 +1859,7 @@ namespace elsa_b200
             unsigned* dViewAxes_ = nullptr;
             RayWindow* dWindows_ = nullptr;
             float2* dCheckpoints_ = nullptr;
-            std::unique_ptr<DeviceBuffer> rows_, columns_; // 2D: the forward's padded image copies
+            std::unique_ptr<StreamScratch> lines_; // 2D: the forward's padded image copies
             int cpStride_ = 0;
             int cpdShift_ = 4; // checkpoint slabs of 2^cpdShift_ planes (3D)
 

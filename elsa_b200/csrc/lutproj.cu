@@ -97,7 +97,7 @@ namespace elsa_b200
                 stride_[fast_] = 1, stride_[0] = vol.n[fast_];
                 stride_[3 - fast_] = static_cast<int64_t>(vol.n[fast_]) * vol.n[0];
                 try {
-                    copy_ = std::make_unique<DeviceBuffer>(sizeof(float) *
+                    copy_ = std::make_unique<StreamScratch>(sizeof(float) *
                                                            static_cast<size_t>(domainSize_));
                     second_ = std::make_unique<DeviceBuffer>(sizeof(unsigned long long) *
                                                              static_cast<size_t>(domainSize_));
@@ -110,10 +110,13 @@ namespace elsa_b200
 
             void forward(const float* x, float* y, cudaStream_t s) override
             {
-                if (copy_)
-                    launchLayoutCopy(x, vol_, fast_, stride_, copy_->as<float>(), s);
+                std::unique_ptr<StreamScratch::Lease> copy;
+                if (copy_) {
+                    copy = std::make_unique<StreamScratch::Lease>(*copy_, s);
+                    launchLayoutCopy(x, vol_, fast_, stride_, copy->as<float>(), s);
+                }
                 launchLutForward(dPoses_, det_, lp_, lut_.as<float>(),
-                                 layouts(x, copy_ ? copy_->as<float>() : nullptr), y, s);
+                                 layouts(x, copy ? copy->as<float>() : nullptr), y, s);
                 ELSA_LAUNCH_CHECK("lutForwardKernel");
             }
 
@@ -156,7 +159,8 @@ namespace elsa_b200
 
             int fast_ = 1;        // contiguous axis of the copy for rays that lead along x
             int64_t stride_[3];   // its strides
-            std::unique_ptr<DeviceBuffer> copy_, second_; // volume copy, second set of sums
+            std::unique_ptr<StreamScratch> copy_;   // the volume copy
+            std::unique_ptr<DeviceBuffer> second_; // a second set of sums
             DeviceBuffer lut_, absMax_, acc_;
             LutProjParams lp_{};
         };

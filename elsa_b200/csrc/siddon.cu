@@ -931,7 +931,7 @@ namespace elsa_b200
                         fast_[g] = 0;
                     } else if (f != 0 && !copies_[f]) {
                         try {
-                            copies_[f] = std::make_unique<DeviceBuffer>(
+                            copies_[f] = std::make_unique<StreamScratch>(
                                 sizeof(float) * static_cast<size_t>(domainSize_));
                         } catch (const Error&) { // no room: the volume itself serves
                             cudaGetLastError();
@@ -953,17 +953,19 @@ namespace elsa_b200
                     layouts.stride[g][0] = 1, layouts.stride[g][1] = vol_.n[0];
                     layouts.stride[g][2] = plane;
                 }
+                std::unique_ptr<StreamScratch::Lease> copies[3];
                 for (int f = 1; f < vol_.dim; ++f) {
                     if (!copies_[f])
                         continue;
+                    copies[f] = std::make_unique<StreamScratch::Lease>(*copies_[f], s);
                     // axis f contiguous, then x, then the third axis
                     const int64_t nf = vol_.n[f];
                     int64_t stride[3];
                     stride[f] = 1, stride[0] = nf, stride[3 - f] = nf * vol_.n[0];
-                    launchLayoutCopy(x, vol_, f, stride, copies_[f]->as<float>(), s);
+                    launchLayoutCopy(x, vol_, f, stride, copies[f]->as<float>(), s);
                     for (int g = 0; g < vol_.dim; ++g)
                         if (fast_[g] == f) {
-                            layouts.base[g] = copies_[f]->as<float>();
+                            layouts.base[g] = copies[f]->as<float>();
                             std::copy(stride, stride + 3, layouts.stride[g]);
                         }
                 }
@@ -1374,7 +1376,7 @@ namespace elsa_b200
             CurvedDetector curved_;
             std::unique_ptr<DeviceBuffer> rays_, cpState_, cpVoxel_, viewAxes_, windows_;
             std::array<int, 3> fast_{{0, 0, 0}};     // contiguous axis per driving axis (forward)
-            std::unique_ptr<DeviceBuffer> copies_[3]; // volume copies with axis 1 or 2 contiguous
+            std::unique_ptr<StreamScratch> copies_[3]; // volume copies with axis 1 or 2 contiguous
             int cpRows_ = 0;
             int classSpacing_ = 0;
             int64_t visits_ = 0;

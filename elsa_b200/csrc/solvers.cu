@@ -99,6 +99,37 @@ namespace elsa_b200
             cudaFree(ptr_);
     }
 
+    StreamScratch::Lease::Lease(StreamScratch& scratch, cudaStream_t s) : stream_(s)
+    {
+        {
+            std::lock_guard<std::mutex> lock(scratch.mutex_);
+            // (the per-thread default stream is one handle for many streams)
+            if (!scratch.claimed_ && s != cudaStreamPerThread) {
+                scratch.claimed_ = true;
+                scratch.home_ = s;
+            }
+            if (scratch.claimed_ && s == scratch.home_) {
+                ptr_ = scratch.initial();
+                return;
+            }
+        }
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capture) != cudaSuccess)
+            cudaGetLastError();
+        if (capture != cudaStreamCaptureStatusNone) {
+            ptr_ = scratch.initial();
+            return;
+        }
+        ELSA_CUDA(cudaMallocAsync(&ptr_, scratch.bytes(), s));
+        own_ = true;
+    }
+
+    StreamScratch::Lease::~Lease()
+    {
+        if (own_)
+            cudaFreeAsync(ptr_, stream_);
+    }
+
     SolverWorkspace::SolverWorkspace(int64_t domain, int64_t range)
         : vol0(sizeof(float) * domain), vol1(sizeof(float) * domain),
           vol2(sizeof(float) * domain), vol3(sizeof(float) * domain),

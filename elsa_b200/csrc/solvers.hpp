@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
 #include "projector.hpp"
@@ -30,6 +31,45 @@ namespace elsa_b200
     private:
         void* ptr_ = nullptr;
         size_t bytes_ = 0;
+    };
+
+    // Scratch that a forward writes and reads within one call. The first stream that asks owns the
+    // buffer (its calls are ordered); calls on other streams get stream-ordered memory of their
+    // own, so that they do not share it. A captured call takes the buffer too: its graph, like the
+    // solver session it belongs to, is to be ordered with the projector's other calls.
+    class StreamScratch
+    {
+    public:
+        explicit StreamScratch(size_t bytes) : buffer_(bytes) {}
+
+        class Lease
+        {
+        public:
+            Lease(StreamScratch& scratch, cudaStream_t s);
+            ~Lease();
+            Lease(const Lease&) = delete;
+            Lease& operator=(const Lease&) = delete;
+            template <typename T>
+            T* as() const
+            {
+                return static_cast<T*>(ptr_);
+            }
+            bool own() const { return own_; } // memory of this call, not initialised
+
+        private:
+            void* ptr_ = nullptr;
+            bool own_ = false;
+            cudaStream_t stream_;
+        };
+
+        size_t bytes() const { return buffer_.bytes(); }
+        void* initial() const { return buffer_.as<void>(); } // to initialise the buffer
+
+    private:
+        DeviceBuffer buffer_;
+        std::mutex mutex_;
+        bool claimed_ = false;
+        cudaStream_t home_ = nullptr;
     };
 
     // Scratch for one solver run: four volume-sized and two sinogram-sized float buffers, the

@@ -141,3 +141,28 @@ def test_voxel_adjoint_same_footprints_at_size(cuda, oracle):
     fast = _apply(cuda, proj, y, True)
     proj.set_knob(elsa_b200.KNOB_EXACT_WEIGHTS, 1)
     assert rel_l2(fast, _apply(cuda, proj, y, True)) <= 5e-7
+
+
+@pytest.mark.parametrize("kind,vol,det", [("JOSEPH", (300, 280), [401]), ("JOSEPH", (120, 100), [150]),
+                                          ("SIDDON", (60, 50, 70), [90, 80]),
+                                          ("BLOB", (40, 50, 45), [60, 70]),
+                                          ("RAY_BLOB", (24, 20, 28), [40, 30])])
+def test_forwards_on_two_streams(cuda, oracle, kind, vol, det):
+    """The forwards' scratch is not shared between streams."""
+    import elsa_b200
+    torch = cuda
+    poses, det, x, _ = _problem(oracle, vol, 40, det)
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    xs = [torch.from_numpy(x).cuda() * (k + 1) for k in range(2)]
+    ref = [_apply(torch, proj, v.cpu().numpy(), False) for v in xs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[torch.empty(proj.range_size, device="cuda") for _ in range(4)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for i in range(4):
+        for k, s in enumerate(streams):
+            proj.apply_ptr(xs[k].data_ptr(), outs[k][i].data_ptr(), s.cuda_stream)
+    torch.cuda.synchronize()
+    for k in range(2):
+        for o in outs[k]:
+            # (the voxel forward's atomics reorder its sums)
+            assert rel_l2(o.cpu().numpy(), ref[k]) <= (1e-6 if kind == "BLOB" else 0.0)
