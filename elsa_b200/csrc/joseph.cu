@@ -1218,7 +1218,8 @@ namespace elsa_b200
         // blocks; their rays start and end in more tiles).
         using Adjoint2dLarge = Adjoint2dConfig<64, 4>;
         using Adjoint2dSmall = Adjoint2dConfig<32, 8>;
-                constexpr int kSmallImage = 256 * 256; // pixels (512^2: 0.504 ms with tiles of 32, 0.514 of 64)
+                constexpr int kSmallImage = 256 * 256; // pixels (512^2 adjoint: 0.504 ms with tiles of 32,
+                                               // 0.514 of 64, which need half the checkpoints)
 
         class JosephProjector final : public Projector
         {

@@ -458,7 +458,8 @@ namespace elsa_b200
                             dist = root2(sq, h);
                         else
                             dist = make_float2(sqrtf(sq.x), sqrtf(sq.y));
-                        f(word, i + 1 < to[I], lutValue2(tab, lp.lutN, lp.radius, lp.exactInv, dist, zero));
+                        f(word, i + 1 < to[I],
+                          lutValue2(tab, lp.lutN, lp.radius, lp.exactInv, dist, zero));
                     }
                 }
             }
@@ -483,9 +484,9 @@ namespace elsa_b200
                 body(std::integral_constant<int, DIM == 3 ? 2 : 1>{});
         }
 
-        // Forward, one thread per ray. Bound by issue (about 50
-        // instructions per voxel; 64^3 / 60 views / 96^2, forward and adjoint: 10.8 ms with
-        // one voxel at a time on the x-fastest volume, now 4.20).
+        // Forward, one thread per ray. Bound by issue (about 50 instructions per voxel; 64^3 / 60
+        // views / 96^2, forward and adjoint: 10.8 ms with one voxel at a time on the x-fastest
+        // volume, now 4.20).
         template <int DIM>
         __global__ void __launch_bounds__(128)
             lutForwardKernel(const float* __restrict__ poses, DetectorShape det,
@@ -553,8 +554,8 @@ namespace elsa_b200
             withLead<DIM>(d, [&](auto lead) {
                 constexpr int L = decltype(lead)::value;
                 constexpr int I = DIM == 2 ? 1 - L : (L == 2 ? 1 : 2);
-                auto* acc =
-                    const_cast<unsigned long long*>(static_cast<const unsigned long long*>(layouts.base[L]));
+                auto* acc = const_cast<unsigned long long*>(
+                    static_cast<const unsigned long long*>(layouts.base[L]));
                 const int64_t next = layouts.stride[L][I];
                 // scale is a power of two: the product is exact in float too, where that holds it
                 // (a result that is subnormal rounds to 0 either way)

@@ -130,9 +130,9 @@ namespace elsa_b200
         // (about 25 instructions per visit) once neighbouring lanes read neighbouring words: with
         // every ray on the x-fastest volume, a warp whose rays drive along x read 32 sectors per
         // visit and the load pipe took the time (171 x 200 x 149 voxels, 240 views of
-        // 250 x 231: 3.62 ms, now 2.69). The bounds test counts the steps left along each axis, so a visit updates
-        // one word offset instead of three voxel indices and a 64-bit one. Offset: unsigned below
-        // 2^32 words, else int64_t.
+        // 250 x 231: 3.62 ms, now 2.69). The bounds test counts the steps left along each axis, so
+        // a visit updates one word offset instead of three voxel indices and a 64-bit one. Offset:
+        // unsigned below 2^32 words, else int64_t.
         template <int DIM, typename Offset>
         __global__ void __launch_bounds__(kMaxForwardThreads)
             siddonForwardKernel(const SiddonRay* __restrict__ rays, int64_t nrays,
@@ -683,7 +683,8 @@ namespace elsa_b200
             float tEntry = cp.w;
             // the walk stays inside the volume and the slab: along G the two tests are one,
             // kLo <= cg < min(kLo + kSlab, n_G)
-            const unsigned nA = static_cast<unsigned>(a == 0 ? vol.n[0] : (a == 1 ? vol.n[1] : vol.n[2]));
+            const unsigned nA =
+                static_cast<unsigned>(a == 0 ? vol.n[0] : (a == 1 ? vol.n[1] : vol.n[2]));
             const unsigned nB = static_cast<unsigned>(b == 1 ? vol.n[1] : vol.n[2]);
             const int nG = G == 0 ? vol.n[0] : (G == 1 ? vol.n[1] : vol.n[2]);
             const unsigned spanG = static_cast<unsigned>(min(kLo + kSlab, nG) - kLo);
