@@ -193,7 +193,7 @@ elsa_status elsa_projector_wait_test(elsa_projector* projector, int64_t waitCycl
  * ProjectVoxelsCUDA.cu:21-239). */
 #define ELSA_KNOB_FORWARD_THREADS 0 /* rays per block of a thread-per-ray forward (Siddon, 2D Joseph) */
 #define ELSA_KNOB_ADJOINT_CHUNKS 1  /* view chunks of a brick-owner adjoint (Joseph, Siddon) */
-#define ELSA_KNOB_ADJOINT_THREADS 2 /* voxels per block of a thread-per-voxel adjoint (blob, B-spline) */
+#define ELSA_KNOB_ADJOINT_THREADS 2 /* threads per block of a voxel-driven adjoint (blob, B-spline) */
 /* Adjoint scheme of Joseph (matched adjoint), Siddon and BinaryMethod: 0 = deterministic
  * brick-owner kernel (bit-reproducible), 1 = thread-per-ray atomic scatter, the reference's own
  * scheme (SiddonsMethod.cpp:119 `omp atomic`, TraverseSiddonsCUDA.cu atomicAdd): the same sums
@@ -201,14 +201,14 @@ elsa_status elsa_projector_wait_test(elsa_projector* projector, int64_t waitCycl
  * the brick owner exists for the geometry (a valid class spacing) and its checkpoint tables
  * (20 bytes per ray and 16-plane slab, about 20 GB at 256^3 / 360 x 384^2) take at most a quarter
  * of the device's memory and half of the free memory at creation, else 1. At 256^3 the Siddon
- * brick owner takes 1.22x the scatter's time. */
+ * brick owner takes 0.94x the scatter's time (30.8 ms, 32.6 ms). */
 #define ELSA_KNOB_ADJOINT_SCATTER 3
 /* Weights of the voxel projectors' adjoint (blob, B-spline and their phase-contrast forms):
  * 0 = the forward's weights (distance as n2 * rsqrt(n2), scaling applied as a multiplication by
  * 1 / s, the table lerp as one fma; within a few ulp of the reference's, and forward and adjoint
  * then use the same weights), 1 = the reference's float operations (VoxelComputation.h:55-185),
- * the adjoint bit-identical to elsa's CPU loop. Default 0 (1.4x faster). Either way the adjoint
- * is deterministic. */
+ * the adjoint bit-identical to elsa's CPU loop. Default 0 (3.1x faster: 128^3
+ * blob 7.8 ms, 24.0 ms). Either way the adjoint is deterministic. */
 #define ELSA_KNOB_EXACT_WEIGHTS 4
 /* Planes per checkpoint slab of the 3D Joseph matched adjoint: 16, 32, 64 or 128. The adjoint
  * replays every ray from its exact accumulated position at the slab's first sample (8 bytes per
