@@ -848,7 +848,7 @@ namespace elsa_b200
             const SumChunksEntry E = e[blockIdx.y];
             for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
                  v < E.nvox; v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-                float s = E.partial[v];
+                float s = E.chunks > 0 ? E.partial[v] : 0.0f;
                 for (int c = 1; c < E.chunks; ++c)
                     s = s + E.partial[c * E.nvox + v];
                 E.x[v] = s;
@@ -1530,6 +1530,10 @@ namespace elsa_b200
                     return;
                 }
                 if (vol_.dim == 3) {
+                    if (axisPartials_ == 0) { // no ray meets the volume: nothing else writes x
+                        ELSA_CUDA(cudaMemsetAsync(x, 0, sizeof(float) * domainSize_, s));
+                        return;
+                    }
                     const int used = usedChunks();
                     float* out = axisPartials_ > 1 ? partial_->as<float>() : x;
                     launchAxisChunks(0, used, y, out, s);
@@ -1562,7 +1566,7 @@ namespace elsa_b200
             {
                 if (batch <= 0)
                     return;
-                if (fast_ || scatter_ || vol_.dim != 3) {
+                if (fast_ || scatter_ || vol_.dim != 3 || axisPartials_ == 0) {
                     Projector::adjointBatch(y, ys, x, xs, batch, s);
                     return;
                 }
@@ -2007,7 +2011,8 @@ namespace elsa_b200
 
         public:
             // This operator's share of a batched adjoint (planJosephAdjointMany): its axis-brick
-            // jobs keyed by (grid, column axis), and its chunk sum (chunks <= 1: none).
+            // jobs keyed by (grid, column axis), and its chunk sum (one partial volume: none; no
+            // partial volume, as no ray meets the volume: a sum of none, which writes zeros).
             bool batchable() const
             {
                 return vol_.dim == 3 && !fast_ && !scatter_ && dCheckpoints_ != nullptr;
@@ -2022,9 +2027,9 @@ namespace elsa_b200
                         continue;
                     jobs[2 * g + (G.ub ? 1 : 0)].push_back(axisJob(g, y, out));
                 }
-                if (axisPartials_ > 1)
-                    sums.push_back(SumChunksEntry{partial_->as<float>(), axisPartials_,
-                                                  domainSize_, x});
+                if (axisPartials_ != 1)
+                    sums.push_back(SumChunksEntry{axisPartials_ > 1 ? out : nullptr,
+                                                  axisPartials_, domainSize_, x});
             }
 
         private:

@@ -1007,6 +1007,10 @@ namespace elsa_b200
                 if (!cpState_)
                     throw Error(ELSA_ERROR_LOGIC, "SiddonsMethod: brick-owner adjoint not built");
                 if (vol_.dim == 3) {
+                    if (axisPartials_ == 0) { // no ray meets the volume: nothing else writes x
+                        ELSA_CUDA(cudaMemsetAsync(x, 0, sizeof(float) * domainSize_, s));
+                        return;
+                    }
                     float* out = axisPartials_ > 1 ? partial_->as<float>() : x;
                     const int per = (det_.np + adjointChunks_ - 1) / adjointChunks_;
                     for (int g = 0; g < 3; ++g) {

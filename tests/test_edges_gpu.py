@@ -166,3 +166,67 @@ def test_forwards_on_two_streams(cuda, oracle, kind, vol, det):
         for o in outs[k]:
             # (the voxel forward's atomics reorder its sums)
             assert rel_l2(o.cpu().numpy(), ref[k]) <= (1e-6 if kind == "BLOB" else 0.0)
+
+
+@pytest.mark.parametrize("vol", [(20, 17, 23), (40, 33)])
+@pytest.mark.parametrize("kind", ["JOSEPH", "SIDDON", "BINARY", "BLOB", "RAY_BLOB"])
+def test_no_ray_meets_the_volume(cuda, kind, vol):
+    """A detector far off the volume: zeros in both directions, written over what the output held,
+    through every entry point."""
+    import elsa_b200
+    torch = cuda
+    dim, n = len(vol), max(vol)
+    det = [30, 24, 6][:dim - 1] + [6]
+    origin = [0.5 * v for v in vol]
+    sino = [0.5 * v for v in det[:-1]]
+    one = [1.0] * dim
+    if dim == 3:
+        poses = [elsa_b200.pose_3d(5.0 * n, 1.5 * n, one, origin, one, sino + [0.0], g,
+                                   pp_offset=(30.0 * n, 0.0)) for g in np.linspace(0.0, 3.0, 6)]
+    else:
+        poses = [elsa_b200.pose_2d(5.0 * n, 1.5 * n, g, one, origin, [1.0, 1.0], sino + [0.0],
+                                   pp_offset=30.0 * n) for g in np.linspace(0.0, 3.0, 6)]
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det,
+                               np.concatenate(poses))
+    rng = np.random.default_rng(2)
+    x = rng.uniform(1, 2, int(np.prod(vol))).astype(np.float32)
+    y = rng.uniform(1, 2, int(np.prod(det))).astype(np.float32)
+    assert not _apply(torch, proj, x, False).any()
+    scatters = [0, 1] if kind in ("JOSEPH", "SIDDON", "BINARY") else [None]
+    for scatter in scatters:
+        if scatter is not None:
+            proj.set_knob(elsa_b200.KNOB_ADJOINT_SCATTER, scatter)
+        assert not _apply(torch, proj, y, True).any()
+        assert not proj.apply_adjoint_host(y).any()
+        s = torch.cuda.current_stream().cuda_stream
+        ys = torch.from_numpy(np.stack([y, y])).cuda()
+        xs = torch.full((2, proj.domain_size), float("nan"), device="cuda")
+        proj.apply_adjoint_batch_ptr(ys.data_ptr(), proj.range_size, xs.data_ptr(),
+                                     proj.domain_size, 2, s)
+        torch.cuda.synchronize()
+        assert not xs.cpu().numpy().any()
+
+
+def test_batched_solve_with_an_operator_that_meets_nothing(cuda, oracle):
+    """Its normal equations are 0 x = 0; the other instances are not disturbed."""
+    import elsa_b200
+    torch = cuda
+    n = 24
+    vol, one = (n, n, n), [1.0] * 3
+    poses, det, _, y = _problem(oracle, vol, 8, [36, 36])
+    off = np.concatenate([elsa_b200.pose_3d(5.0 * n, 1.5 * n, one, [0.5 * n] * 3, one,
+                                            [18.0, 18.0, 0.0], g, pp_offset=(30.0 * n, 0.0))
+                          for g in np.linspace(0.0, 3.0, 8)])
+    ops = [elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, p) for p in (poses, off)]
+    b = [torch.from_numpy(y).cuda() for _ in ops]
+    xs = [torch.zeros(n ** 3, device="cuda") for _ in ops]
+    s = torch.cuda.current_stream().cuda_stream
+    batch = elsa_b200.BatchCGNE(ops, [t.data_ptr() for t in b], [t.data_ptr() for t in xs], s)
+    batch.iterate(1, s)
+    single = torch.zeros(n ** 3, device="cuda")
+    solver = elsa_b200.Solver(elsa_b200.SOLVER_CGNE, ops[0], b[0].data_ptr(), single.data_ptr(),
+                              stream=s)
+    solver.iterate(1, s)
+    torch.cuda.synchronize()
+    assert torch.equal(xs[0], single)
+    assert not batch.squared_residuals(s)[1] > 0.0  # 0 / 0 afterwards, as in a solve of its own
