@@ -230,3 +230,48 @@ def test_batched_solve_with_an_operator_that_meets_nothing(cuda, oracle):
     torch.cuda.synchronize()
     assert torch.equal(xs[0], single)
     assert not batch.squared_residuals(s)[1] > 0.0  # 0 / 0 afterwards, as in a solve of its own
+
+
+VOXEL_KINDS = [("blob", (2.0, 10.83, 2)), ("bspline", (3,)), ("phase_blob", (2.0, 10.83, 2)),
+               ("phase_bspline", (3,))]
+VOXEL_CODES = {"blob": 2, "bspline": 3, "phase_blob": 4, "phase_bspline": 5}
+
+
+def _voxel_reference(oracle, kind, params, dim):
+    if kind.endswith("blob"):
+        return oracle.voxel_lut(kind, dim, *params)
+    return oracle.voxel_lut(kind, dim, order=params[0])
+
+
+@pytest.mark.parametrize("kind,params", VOXEL_KINDS)
+@pytest.mark.parametrize("s2c,c2d", [(-100.0, 300.0), (-40.0, 90.0), (-90.0, 30.0), (6.0, 90.0)])
+@pytest.mark.parametrize("vol,det", [((13, 21, 9), [17, 12]), ((30, 23), [41])])
+def test_voxel_source_in_front_or_inside(cuda, oracle, vol, det, s2c, c2d, kind, params):
+    """A volume behind the source projects as well (quotients of two negative numbers), also with
+    a negative source-detector distance, and around a source inside the volume."""
+    import elsa_b200
+    poses, det = elsa_b200.circle_trajectory(vol, 5, 300.0, s2c, c2d, det)
+    rng = np.random.default_rng(4)
+    x = rng.uniform(0, 1, int(np.prod(vol))).astype(np.float32)
+    y = rng.uniform(0, 1, int(np.prod(det))).astype(np.float32)
+    proj = elsa_b200.Projector(VOXEL_CODES[kind], vol, det, poses,
+                               tuple(map(float, params)) + (1,))
+    args = (vol, det, poses, *_voxel_reference(oracle, kind, params, len(vol)), 1)
+    assert rel_l2(_apply(cuda, proj, x, False), oracle.voxel_project(False, x, *args)) <= PARITY
+    assert rel_l2(_apply(cuda, proj, y, True), oracle.voxel_project(True, y, *args)) <= PARITY
+
+
+@pytest.mark.parametrize("vol,det", [((13, 21, 9), [17, 12]), ((30, 23), [41])])
+def test_voxel_pose_of_nan(cuda, oracle, vol, det):
+    """A pose that is not a number spoils its own view and no other."""
+    import elsa_b200
+    poses, det, x, _ = _problem(oracle, vol, 3, det)
+    size = int(np.prod(det[:-1]))
+    ref = _apply(cuda, elsa_b200.Projector(elsa_b200.PROJECTOR_BLOB, vol, det, poses), x, False)
+    poses = np.array(poses, np.float32).reshape(3, -1)
+    poses[1] = np.nan
+    got = _apply(cuda, elsa_b200.Projector(elsa_b200.PROJECTOR_BLOB, vol, det, poses.ravel()), x,
+                 False)
+    for view in (0, 2):
+        part = slice(view * size, (view + 1) * size)
+        assert rel_l2(got[part], ref[part]) <= 1e-6  # the forward's atomics reorder its sums
