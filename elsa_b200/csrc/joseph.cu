@@ -1446,7 +1446,7 @@ namespace elsa_b200
                 cudaFree(dCheckpoints_);
             }
 
-            void forward(const float* x, float* y, cudaStream_t s) override
+            void doForward(const float* x, float* y, cudaStream_t s) override
             {
                 if (tma_)
                     tma_->forward(x, y, s);
@@ -1488,7 +1488,7 @@ namespace elsa_b200
                 ELSA_LAUNCH_CHECK("josephForward2dKernel");
             }
 
-            void adjoint(const float* y, float* x, cudaStream_t s) override
+            void doAdjoint(const float* y, float* x, cudaStream_t s) override
             {
                 if (fast_) {
                     // the sinogram into the layered array (JosephsMethodCUDA.cpp:234-240 copies
@@ -1552,22 +1552,22 @@ namespace elsa_b200
             // Batched applies (3D matched operator): one launch per kernel for all volumes,
             // sharing the ray tables; every batch element is computed exactly as by a single
             // apply (same kernels, chunks and summation order).
-            void forwardBatch(const float* x, int64_t xs, float* y, int64_t ys, int batch,
-                              cudaStream_t s) override
+            void doForwardBatch(const float* x, int64_t xs, float* y, int64_t ys, int batch,
+                                cudaStream_t s) override
             {
                 if (!tma_) {
-                    Projector::forwardBatch(x, xs, y, ys, batch, s);
+                    Projector::doForwardBatch(x, xs, y, ys, batch, s);
                     return;
                 }
                 tma_->forwardBatch(x, xs, y, ys, batch, s);
             }
-            void adjointBatch(const float* y, int64_t ys, float* x, int64_t xs, int batch,
-                              cudaStream_t s) override
+            void doAdjointBatch(const float* y, int64_t ys, float* x, int64_t xs, int batch,
+                                cudaStream_t s) override
             {
                 if (batch <= 0)
                     return;
                 if (fast_ || scatter_ || vol_.dim != 3 || axisPartials_ == 0) {
-                    Projector::adjointBatch(y, ys, x, xs, batch, s);
+                    Projector::doAdjointBatch(y, ys, x, xs, batch, s);
                     return;
                 }
                 const int used = usedChunks();

@@ -108,7 +108,7 @@ namespace elsa_b200
                                      sizeof(float) * lut.values.size(), cudaMemcpyHostToDevice));
             }
 
-            void forward(const float* x, float* y, cudaStream_t s) override
+            void doForward(const float* x, float* y, cudaStream_t s) override
             {
                 std::unique_ptr<StreamScratch::Lease> copy;
                 if (copy_) {
@@ -120,7 +120,7 @@ namespace elsa_b200
                 ELSA_LAUNCH_CHECK("lutForwardKernel");
             }
 
-            void adjoint(const float* y, float* x, cudaStream_t s) override
+            void doAdjoint(const float* y, float* x, cudaStream_t s) override
             {
                 auto* acc = acc_.as<unsigned long long>();
                 auto* second = second_ ? second_->as<unsigned long long>() : nullptr;

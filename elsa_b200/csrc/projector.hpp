@@ -11,6 +11,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -66,21 +67,31 @@ namespace elsa_b200
     {
     public:
         virtual ~Projector();
-        virtual void forward(const float* x, float* y, cudaStream_t stream) = 0;
-        virtual void adjoint(const float* y, float* x, cudaStream_t stream) = 0;
-        // `batch` applies on x + b xStride -> y + b yStride (adjoint: y + b yStride ->
-        // x + b xStride), each exactly as a single apply computes it; the default loops.
-        virtual void forwardBatch(const float* x, int64_t xStride, float* y, int64_t yStride,
-                                  int batch, cudaStream_t stream)
+        // An apply is several launches that pass data through scratch of the projector. The mutex
+        // keeps those of one call together, so that host threads may share a stream.
+        void forward(const float* x, float* y, cudaStream_t stream)
         {
-            for (int b = 0; b < batch; ++b)
-                forward(x + b * xStride, y + b * yStride, stream);
+            const std::lock_guard<std::mutex> lock(enqueue_);
+            doForward(x, y, stream);
         }
-        virtual void adjointBatch(const float* y, int64_t yStride, float* x, int64_t xStride,
-                                  int batch, cudaStream_t stream)
+        void adjoint(const float* y, float* x, cudaStream_t stream)
         {
-            for (int b = 0; b < batch; ++b)
-                adjoint(y + b * yStride, x + b * xStride, stream);
+            const std::lock_guard<std::mutex> lock(enqueue_);
+            doAdjoint(y, x, stream);
+        }
+        // `batch` applies on x + b xStride -> y + b yStride (adjoint: y + b yStride ->
+        // x + b xStride), each exactly as a single apply computes it.
+        void forwardBatch(const float* x, int64_t xStride, float* y, int64_t yStride, int batch,
+                          cudaStream_t stream)
+        {
+            const std::lock_guard<std::mutex> lock(enqueue_);
+            doForwardBatch(x, xStride, y, yStride, batch, stream);
+        }
+        void adjointBatch(const float* y, int64_t yStride, float* x, int64_t xStride, int batch,
+                          cudaStream_t stream)
+        {
+            const std::lock_guard<std::mutex> lock(enqueue_);
+            doAdjointBatch(y, yStride, x, xStride, batch, stream);
         }
 
         int64_t domainSize() const { return domainSize_; }
@@ -150,6 +161,21 @@ namespace elsa_b200
     protected:
         Projector(int kind, const VolumeShape& vol, const DetectorShape& det,
                   const std::vector<PoseRecord>& poses);
+        virtual void doForward(const float* x, float* y, cudaStream_t stream) = 0;
+        virtual void doAdjoint(const float* y, float* x, cudaStream_t stream) = 0;
+        // (the default loops)
+        virtual void doForwardBatch(const float* x, int64_t xStride, float* y, int64_t yStride,
+                                    int batch, cudaStream_t stream)
+        {
+            for (int b = 0; b < batch; ++b)
+                doForward(x + b * xStride, y + b * yStride, stream);
+        }
+        virtual void doAdjointBatch(const float* y, int64_t yStride, float* x, int64_t xStride,
+                                    int batch, cudaStream_t stream)
+        {
+            for (int b = 0; b < batch; ++b)
+                doAdjoint(y + b * yStride, x + b * xStride, stream);
+        }
         int kind_;
         VolumeShape vol_;
         DetectorShape det_;
@@ -157,6 +183,9 @@ namespace elsa_b200
         int64_t domainSize_ = 0, rangeSize_ = 0;
         std::vector<PoseRecord> poses_;
         float* dPoses_ = nullptr;
+
+    private:
+        std::mutex enqueue_;
     };
 
     std::unique_ptr<Projector> makeJosephProjector(const VolumeShape& vol,

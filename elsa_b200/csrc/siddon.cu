@@ -950,7 +950,7 @@ namespace elsa_b200
                 }
             }
 
-            void forward(const float* x, float* y, cudaStream_t s) override
+            void doForward(const float* x, float* y, cudaStream_t s) override
             {
                 const int64_t nrays = rangeSize_;
                 const unsigned blocks =
@@ -988,7 +988,7 @@ namespace elsa_b200
                 ELSA_LAUNCH_CHECK("siddonForwardKernel");
             }
 
-            void adjoint(const float* y, float* x, cudaStream_t s) override
+            void doAdjoint(const float* y, float* x, cudaStream_t s) override
             {
                 if (scatter_) {
                     const int64_t nrays = rangeSize_;

@@ -258,10 +258,12 @@ elsa_status elsa_tune_cache_get(const char* key, int32_t* values, int32_t* found
 /* y = A x on device buffers. Replaces LinearOperator::apply(x, Ax), core/LinearOperator.cpp:94-98
  * -> XrayProjector::applyImpl -> JosephsMethodCUDA::forward, JosephsMethodCUDA.cpp:132-214.
  * Asynchronous on `stream`.
- * Concurrency: a projector owns device scratch that its applies write (the TMA forward's
- * permuted copies of x, the adjoint's per-view-chunk partial volumes, staging buffers of the
- * host-buffer entry points). Applies of ONE projector must therefore be ordered: issue them on
- * one stream, or order the streams with events. Different projectors (also of the same geometry)
+ * Concurrency: a projector owns device scratch that its applies write (the 3D Joseph forward's
+ * permuted copies of x, the adjoints' per-view-chunk partial volumes and fixed-point sums, staging
+ * buffers of the host-buffer entry points). Applies of ONE projector must therefore be ordered:
+ * issue them on one stream, or order the streams with events. Host threads may share that stream
+ * (the launches of one device-buffer apply stay together); calls of the host-buffer entry points
+ * of one projector follow one another. Different projectors (also of the same geometry)
  * may run concurrently on any streams. The reference's CUDA projectors are not reentrant either
  * (they share the device and synchronize it on every call). */
 elsa_status elsa_projector_apply(elsa_projector* projector, const float* x, float* y,

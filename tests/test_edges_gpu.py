@@ -275,3 +275,50 @@ def test_voxel_pose_of_nan(cuda, oracle, vol, det):
     for view in (0, 2):
         part = slice(view * size, (view + 1) * size)
         assert rel_l2(got[part], ref[part]) <= 1e-6  # the forward's atomics reorder its sums
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("kind,vol,det", [("JOSEPH", (120, 100), [150]),
+                                          ("JOSEPH", (40, 36, 44), [60, 60]),
+                                          ("SIDDON", (60, 50, 70), [90, 80]),
+                                          ("BLOB", (40, 50, 45), [60, 70]),
+                                          ("RAY_BLOB", (24, 20, 28), [40, 30])])
+def test_host_threads_on_one_stream(cuda, oracle, kind, vol, det, adjoint):
+    """Host threads that apply one projector on one stream: every result is that of its own
+    input."""
+    import threading
+    import elsa_b200
+    torch = cuda
+    poses, det, x, y = _problem(oracle, vol, 12, det)
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    base = y if adjoint else x
+    count, repeats = 4, 60
+    data = [torch.from_numpy(base * (k + 1)).cuda() for k in range(count)]
+    ref = [_apply(torch, proj, base * np.float32(k + 1), adjoint) for k in range(count)]
+    size = proj.domain_size if adjoint else proj.range_size
+    outs = [torch.empty((repeats, size), device="cuda") for _ in range(count)]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    apply = proj.apply_adjoint_ptr if adjoint else proj.apply_ptr
+    gate, failed = threading.Barrier(count), []
+
+    def work(k):
+        try:
+            gate.wait()
+            for i in range(repeats):
+                apply(data[k].data_ptr(), outs[k][i].data_ptr(), stream.cuda_stream)
+        except Exception as e:  # reported below, in the main thread
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(count)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    # (the voxel forward's atomics and the Siddon scatter reorder their sums)
+    bound = 1e-6 if kind == "BLOB" and not adjoint else 0.0
+    for k in range(count):
+        for got in outs[k].cpu().numpy():
+            assert rel_l2(got, ref[k]) <= bound
