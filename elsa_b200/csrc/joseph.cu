@@ -1462,7 +1462,7 @@ namespace elsa_b200
             void forward2d(const float* x, float* y, cudaStream_t s)
             {
                 const StreamScratch::Lease lines(*lines_, s);
-                if (lines.own()) // the padding
+                if (lines.fresh()) // the padding
                     ELSA_CUDA(cudaMemsetAsync(lines.as<void>(), 0, lines_->bytes(), s));
                 float* rows = lines.as<float>();
                 float* columns = rows + rowWords();

@@ -99,34 +99,90 @@ namespace elsa_b200
             cudaFree(ptr_);
     }
 
+    void* StreamScratch::capturedBuffer(unsigned long long capture, cudaGraph_t graph,
+                                        cudaStream_t s, bool& fresh)
+    {
+        Captured* free = nullptr;
+        for (const auto& c : captured_) {
+            const bool live = c->live && c->live->load();
+            if (live && c->capture == capture && c->stream == s)
+                return c->buffer.as<void>(); // an earlier call of this capture and stream
+            if (!live)
+                free = c.get();
+        }
+        if (!free) {
+            // allocating is allowed while the thread's capture interaction is relaxed
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            ELSA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            try {
+                captured_.push_back(std::make_unique<Captured>(bytes()));
+            } catch (...) {
+                cudaGetLastError();
+                cudaThreadExchangeStreamCaptureMode(&mode);
+                throw;
+            }
+            ELSA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            free = captured_.back().get();
+        }
+        // the graph, and with it every executable made from it, keeps the flag set
+        auto live = std::make_shared<std::atomic<bool>>(true);
+        auto* held = new std::shared_ptr<std::atomic<bool>>(live);
+        cudaUserObject_t object = nullptr;
+        const cudaError_t made = cudaUserObjectCreate(
+            &object, held,
+            [](void* p) {
+                auto* flag = static_cast<std::shared_ptr<std::atomic<bool>>*>(p);
+                (*flag)->store(false);
+                delete flag;
+            },
+            1, cudaUserObjectNoDestructorSync);
+        if (made != cudaSuccess) {
+            delete held;
+            ELSA_CUDA(made);
+        }
+        const cudaError_t kept =
+            cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+        if (kept != cudaSuccess) {
+            cudaUserObjectRelease(object, 1);
+            ELSA_CUDA(kept);
+        }
+        free->capture = capture;
+        free->stream = s;
+        free->live = std::move(live);
+        fresh = true;
+        return free->buffer.as<void>();
+    }
+
     StreamScratch::Lease::Lease(StreamScratch& scratch, cudaStream_t s) : stream_(s)
     {
-        {
-            std::lock_guard<std::mutex> lock(scratch.mutex_);
-            // (the per-thread default stream is one handle for many streams)
-            if (!scratch.claimed_ && s != cudaStreamPerThread) {
-                scratch.claimed_ = true;
-                scratch.home_ = s;
-            }
-            if (scratch.claimed_ && s == scratch.home_) {
-                ptr_ = scratch.initial();
-                return;
-            }
-        }
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &capture) != cudaSuccess)
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long capture = 0;
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamGetCaptureInfo_v2(s, &status, &capture, &graph, nullptr, nullptr) !=
+            cudaSuccess) {
             cudaGetLastError();
-        if (capture != cudaStreamCaptureStatusNone) {
+            status = cudaStreamCaptureStatusNone;
+        }
+        if (status == cudaStreamCaptureStatusActive) {
+            ptr_ = scratch.capturedBuffer(capture, graph, s, fresh_);
+            return;
+        }
+        // (the per-thread default stream is one handle for many streams)
+        if (!scratch.claimed_ && s != cudaStreamPerThread) {
+            scratch.claimed_ = true;
+            scratch.home_ = s;
+        }
+        if (scratch.claimed_ && s == scratch.home_) {
             ptr_ = scratch.initial();
             return;
         }
         ELSA_CUDA(cudaMallocAsync(&ptr_, scratch.bytes(), s));
-        own_ = true;
+        fresh_ = temporary_ = true;
     }
 
     StreamScratch::Lease::~Lease()
     {
-        if (own_)
+        if (temporary_)
             cudaFreeAsync(ptr_, stream_);
     }
 

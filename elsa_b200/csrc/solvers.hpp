@@ -3,9 +3,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
-#include <mutex>
+#include <memory>
 #include <vector>
 
 #include "projector.hpp"
@@ -33,10 +34,11 @@ namespace elsa_b200
         size_t bytes_ = 0;
     };
 
-    // Scratch that a forward writes and reads within one call. The first stream that asks owns the
-    // buffer (its calls are ordered); calls on other streams get stream-ordered memory of their
-    // own, so that they do not share it. A captured call takes the buffer too: its graph, like the
-    // solver session it belongs to, is to be ordered with the projector's other calls.
+    // Scratch that a forward writes and reads within one call (under the projector's mutex). The
+    // first stream that asks owns the buffer (its calls are ordered); calls on other streams get
+    // stream-ordered memory of their own, so that they do not share it. A graph being captured gets
+    // a buffer per stream of the capture, whichever stream it is replayed on later; the buffer
+    // serves another capture once the graph and its executables are destroyed.
     class StreamScratch
     {
     public:
@@ -54,11 +56,12 @@ namespace elsa_b200
             {
                 return static_cast<T*>(ptr_);
             }
-            bool own() const { return own_; } // memory of this call, not initialised
+            bool fresh() const { return fresh_; } // memory that is not initialised
 
         private:
             void* ptr_ = nullptr;
-            bool own_ = false;
+            bool fresh_ = false;
+            bool temporary_ = false;
             cudaStream_t stream_;
         };
 
@@ -66,10 +69,21 @@ namespace elsa_b200
         void* initial() const { return buffer_.as<void>(); } // to initialise the buffer
 
     private:
+        // A buffer of a capture; `live` while its graph or an executable of it exists.
+        struct Captured {
+            explicit Captured(size_t bytes) : buffer(bytes) {}
+            DeviceBuffer buffer;
+            unsigned long long capture = 0;
+            cudaStream_t stream = nullptr;
+            std::shared_ptr<std::atomic<bool>> live;
+        };
+        void* capturedBuffer(unsigned long long capture, cudaGraph_t graph, cudaStream_t s,
+                             bool& fresh);
+
         DeviceBuffer buffer_;
-        std::mutex mutex_;
         bool claimed_ = false;
         cudaStream_t home_ = nullptr;
+        std::vector<std::unique_ptr<Captured>> captured_;
     };
 
     // Scratch for one solver run: four volume-sized and two sinogram-sized float buffers, the

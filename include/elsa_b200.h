@@ -263,8 +263,9 @@ elsa_status elsa_tune_cache_get(const char* key, int32_t* values, int32_t* found
  * buffers of the host-buffer entry points). Applies of ONE projector must therefore be ordered:
  * issue them on one stream, or order the streams with events. Host threads may share that stream
  * (the launches of one device-buffer apply stay together); calls of the host-buffer entry points
- * of one projector follow one another. Different projectors (also of the same geometry)
- * may run concurrently on any streams. The reference's CUDA projectors are not reentrant either
+ * of one projector follow one another. The launches of a graph that captured applies are ordered
+ * like the applies themselves; the projector outlives the graph. Different projectors (also of
+ * the same geometry) may run concurrently on any streams. The reference's CUDA projectors are not reentrant either
  * (they share the device and synchronize it on every call). */
 elsa_status elsa_projector_apply(elsa_projector* projector, const float* x, float* y,
                                  void* stream);

@@ -322,3 +322,74 @@ def test_host_threads_on_one_stream(cuda, oracle, kind, vol, det, adjoint):
     for k in range(count):
         for got in outs[k].cpu().numpy():
             assert rel_l2(got, ref[k]) <= bound
+
+
+FORWARDS = [("JOSEPH", (300, 280), [401]), ("JOSEPH", (120, 100), [150]),
+            ("SIDDON", (60, 50, 70), [90, 80]), ("BLOB", (40, 50, 45), [60, 70]),
+            ("RAY_BLOB", (24, 20, 28), [40, 30])]
+
+
+@pytest.mark.parametrize("kind,vol,det", FORWARDS)
+def test_captured_forwards_next_to_others(cuda, oracle, kind, vol, det):
+    """Replays of captured forwards next to one another and to applies on the stream that they were
+    captured on: scratch is not shared between them."""
+    import elsa_b200
+    torch = cuda
+    poses, det, x, _ = _problem(oracle, vol, 40, det)
+    make = lambda: elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    proj, other, repeats = make(), make(), 12
+    xs = [torch.from_numpy(x * np.float32(k + 1)).cuda() for k in range(3)]
+    ref = [_apply(torch, other, v.cpu().numpy(), False) for v in xs]
+    outs = torch.zeros((3, 2, proj.range_size), device="cuda")
+    a, b, c = (torch.cuda.Stream() for _ in range(3))
+    torch.cuda.synchronize()
+    proj.apply_ptr(xs[0].data_ptr(), outs[0][0].data_ptr(), a.cuda_stream)
+    graphs = []
+    for k in (1, 2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=a):
+            for i in range(2):  # two calls of one capture
+                proj.apply_ptr(xs[k].data_ptr(), outs[k][i].data_ptr(), a.cuda_stream)
+        graphs.append(g)
+    torch.cuda.synchronize()
+    bound = 1e-6 if kind == "BLOB" else 0.0  # the voxel forward's atomics reorder its sums
+    for _ in range(repeats):
+        outs.zero_()
+        torch.cuda.synchronize()
+        for i in range(2):
+            for s, g in zip((b, c), graphs):
+                with torch.cuda.stream(s):
+                    g.replay()
+            proj.apply_ptr(xs[0].data_ptr(), outs[0][i].data_ptr(), a.cuda_stream)
+        torch.cuda.synchronize()
+        for k in range(3):
+            for got in outs[k].cpu().numpy():
+                assert rel_l2(got, ref[k]) <= bound
+
+
+def test_captures_reuse_scratch(cuda, oracle):
+    """The scratch of a destroyed graph serves the next capture."""
+    import time
+    import elsa_b200
+    torch = cuda
+    vol = (160, 150, 170)
+    poses, det, x, _ = _problem(oracle, vol, 4, [20, 20])
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_SIDDON, vol, det, poses)
+    d = torch.from_numpy(x).cuda()
+    y = torch.empty(proj.range_size, device="cuda")
+    s = torch.cuda.Stream()
+
+    def capture():
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            proj.apply_ptr(d.data_ptr(), y.data_ptr(), s.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        del g
+        time.sleep(0.05)  # (references are dropped asynchronously)
+
+    capture()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(20):
+        capture()
+    assert free - torch.cuda.mem_get_info()[0] <= 4 * 2 * 4 * x.size  # of 20 captures' two copies
