@@ -110,13 +110,15 @@ namespace elsa_b200
 
             void doForward(const float* x, float* y, cudaStream_t s) override
             {
-                std::unique_ptr<StreamScratch::Lease> copy;
+                std::unique_ptr<StreamScratch::Lease> lease;
+                float* copy = nullptr; // (no room: the volume itself serves)
                 if (copy_) {
-                    copy = std::make_unique<StreamScratch::Lease>(*copy_, s);
-                    launchLayoutCopy(x, vol_, fast_, stride_, copy->as<float>(), s);
+                    lease = std::make_unique<StreamScratch::Lease>(*copy_, s, true);
+                    copy = lease->as<float>();
                 }
-                launchLutForward(dPoses_, det_, lp_, lut_.as<float>(),
-                                 layouts(x, copy ? copy->as<float>() : nullptr), y, s);
+                if (copy)
+                    launchLayoutCopy(x, vol_, fast_, stride_, copy, s);
+                launchLutForward(dPoses_, det_, lp_, lut_.as<float>(), layouts(x, copy), y, s);
                 ELSA_LAUNCH_CHECK("lutForwardKernel");
             }
 

@@ -966,7 +966,9 @@ namespace elsa_b200
                 for (int f = 1; f < vol_.dim; ++f) {
                     if (!copies_[f])
                         continue;
-                    copies[f] = std::make_unique<StreamScratch::Lease>(*copies_[f], s);
+                    copies[f] = std::make_unique<StreamScratch::Lease>(*copies_[f], s, true);
+                    if (!copies[f]->as<float>()) // no room: the volume itself serves
+                        continue;
                     // axis f contiguous, then x, then the third axis
                     const int64_t nf = vol_.n[f];
                     int64_t stride[3];

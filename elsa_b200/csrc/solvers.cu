@@ -99,29 +99,75 @@ namespace elsa_b200
             cudaFree(ptr_);
     }
 
-    void* StreamScratch::capturedBuffer(unsigned long long capture, cudaGraph_t graph,
-                                        cudaStream_t s, bool& fresh)
+    namespace
+    {
+        // Allocations and event queries are allowed while some stream is being captured.
+        class RelaxedCapture
+        {
+        public:
+            RelaxedCapture() { ELSA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode_)); }
+            ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+            RelaxedCapture(const RelaxedCapture&) = delete;
+            RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+        private:
+            cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+        };
+    } // namespace
+
+    StreamScratch::Kept::~Kept()
+    {
+        if (done)
+            cudaEventDestroy(done);
+    }
+
+    // The buffer that `stream` uses, one that no call uses any more, or a new one; null where none
+    // can be kept.
+    StreamScratch::Kept* StreamScratch::keptBuffer(unsigned long long stream, bool& fresh)
+    {
+        for (const auto& k : kept_)
+            if (k->stream == stream)
+                return k.get();
+        const RelaxedCapture relaxed;
+        for (const auto& k : kept_) {
+            if (cudaEventQuery(k->done) == cudaSuccess) {
+                k->stream = stream;
+                return k.get();
+            }
+            cudaGetLastError();
+        }
+        constexpr size_t kBuffers = 4, kBytes = size_t(1) << 30;
+        if (kept_.size() >= kBuffers || (!kept_.empty() && kBuffers * bytes() > kBytes))
+            return nullptr;
+        try {
+            auto k = std::make_unique<Kept>(bytes());
+            ELSA_CUDA(cudaEventCreateWithFlags(&k->done, cudaEventDisableTiming));
+            k->stream = stream;
+            kept_.push_back(std::move(k));
+        } catch (const Error&) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        fresh = true;
+        return kept_.back().get();
+    }
+
+    // The buffer of this capture and stream.
+    StreamScratch::Captured& StreamScratch::capturedBuffer(unsigned long long capture,
+                                                           cudaGraph_t graph, cudaStream_t s,
+                                                           bool& fresh)
     {
         Captured* free = nullptr;
         for (const auto& c : captured_) {
             const bool live = c->live && c->live->load();
             if (live && c->capture == capture && c->stream == s)
-                return c->buffer.as<void>(); // an earlier call of this capture and stream
+                return *c; // (of an earlier call)
             if (!live)
                 free = c.get();
         }
         if (!free) {
-            // allocating is allowed while the thread's capture interaction is relaxed
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            ELSA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-            try {
-                captured_.push_back(std::make_unique<Captured>(bytes()));
-            } catch (...) {
-                cudaGetLastError();
-                cudaThreadExchangeStreamCaptureMode(&mode);
-                throw;
-            }
-            ELSA_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            const RelaxedCapture relaxed;
+            captured_.push_back(std::make_unique<Captured>(bytes()));
             free = captured_.back().get();
         }
         // the graph, and with it every executable made from it, keeps the flag set
@@ -150,38 +196,56 @@ namespace elsa_b200
         free->stream = s;
         free->live = std::move(live);
         fresh = true;
-        return free->buffer.as<void>();
+        return *free;
     }
 
-    StreamScratch::Lease::Lease(StreamScratch& scratch, cudaStream_t s) : stream_(s)
+    StreamScratch::Lease::Lease(StreamScratch& scratch, cudaStream_t s, bool optional) : stream_(s)
+    {
+        try {
+            take(scratch);
+        } catch (const Error&) {
+            if (!optional)
+                throw;
+            cudaGetLastError();
+        }
+    }
+
+    void StreamScratch::Lease::take(StreamScratch& scratch)
     {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-        unsigned long long capture = 0;
+        unsigned long long capture = 0, id = 0;
         cudaGraph_t graph = nullptr;
-        if (cudaStreamGetCaptureInfo_v2(s, &status, &capture, &graph, nullptr, nullptr) !=
+        if (cudaStreamGetCaptureInfo_v2(stream_, &status, &capture, &graph, nullptr, nullptr) !=
             cudaSuccess) {
             cudaGetLastError();
             status = cudaStreamCaptureStatusNone;
         }
         if (status == cudaStreamCaptureStatusActive) {
-            ptr_ = scratch.capturedBuffer(capture, graph, s, fresh_);
+            ptr_ = scratch.capturedBuffer(capture, graph, stream_, fresh_).buffer.as<void>();
             return;
         }
-        // (the per-thread default stream is one handle for many streams)
-        if (!scratch.claimed_ && s != cudaStreamPerThread) {
+        ELSA_CUDA(cudaStreamGetId(stream_, &id));
+        if (!scratch.claimed_) {
             scratch.claimed_ = true;
-            scratch.home_ = s;
+            scratch.home_ = id;
         }
-        if (scratch.claimed_ && s == scratch.home_) {
+        if (id == scratch.home_) {
             ptr_ = scratch.initial();
             return;
         }
-        ELSA_CUDA(cudaMallocAsync(&ptr_, scratch.bytes(), s));
+        kept_ = scratch.keptBuffer(id, fresh_);
+        if (kept_) {
+            ptr_ = kept_->buffer.as<void>();
+            return;
+        }
+        ELSA_CUDA(cudaMallocAsync(&ptr_, scratch.bytes(), stream_));
         fresh_ = temporary_ = true;
     }
 
     StreamScratch::Lease::~Lease()
     {
+        if (kept_)
+            cudaEventRecord(kept_->done, stream_);
         if (temporary_)
             cudaFreeAsync(ptr_, stream_);
     }

@@ -34,20 +34,41 @@ namespace elsa_b200
         size_t bytes_ = 0;
     };
 
-    // Scratch that a forward writes and reads within one call (under the projector's mutex). The
-    // first stream that asks owns the buffer (its calls are ordered); calls on other streams get
-    // stream-ordered memory of their own, so that they do not share it. A graph being captured gets
-    // a buffer per stream of the capture, whichever stream it is replayed on later; the buffer
-    // serves another capture once the graph and its executables are destroyed.
+    // Scratch that a forward writes and reads within one call (under the projector's mutex). Calls of
+    // one stream are ordered and share a buffer; other streams have buffers of their own. The first
+    // stream that asks owns the buffer made at creation. Further streams get kept buffers, at most
+    // four (or one where four are more than 1 GiB) at a time, handed on between streams once their
+    // last call is complete, and beyond that stream-ordered memory, which costs far more: the
+    // device's pool returns it to the system at every synchronization (2D Joseph forward at 64^2 / 60
+    // views, each call waited for: 24 us on the first stream, 25 with a kept buffer, 455 so). A graph
+    // being captured gets a buffer per stream of the capture, whichever stream it is replayed on
+    // later; the buffer serves another capture once the graph and its executables are destroyed.
     class StreamScratch
     {
+        struct Kept {
+            explicit Kept(size_t bytes) : buffer(bytes) {}
+            ~Kept();
+            DeviceBuffer buffer;
+            unsigned long long stream = 0; // id of the stream that uses it
+            cudaEvent_t done = nullptr;    // after its last call
+        };
+        // A buffer of a capture; `live` while its graph or an executable of it exists.
+        struct Captured {
+            explicit Captured(size_t bytes) : buffer(bytes) {}
+            DeviceBuffer buffer;
+            unsigned long long capture = 0;
+            cudaStream_t stream = nullptr;
+            std::shared_ptr<std::atomic<bool>> live;
+        };
+
     public:
         explicit StreamScratch(size_t bytes) : buffer_(bytes) {}
 
         class Lease
         {
         public:
-            Lease(StreamScratch& scratch, cudaStream_t s);
+            // optional: without room there is no memory (as() is null) instead of an error
+            Lease(StreamScratch& scratch, cudaStream_t s, bool optional = false);
             ~Lease();
             Lease(const Lease&) = delete;
             Lease& operator=(const Lease&) = delete;
@@ -59,9 +80,11 @@ namespace elsa_b200
             bool fresh() const { return fresh_; } // memory that is not initialised
 
         private:
+            void take(StreamScratch& scratch);
             void* ptr_ = nullptr;
             bool fresh_ = false;
             bool temporary_ = false;
+            Kept* kept_ = nullptr;
             cudaStream_t stream_;
         };
 
@@ -69,20 +92,14 @@ namespace elsa_b200
         void* initial() const { return buffer_.as<void>(); } // to initialise the buffer
 
     private:
-        // A buffer of a capture; `live` while its graph or an executable of it exists.
-        struct Captured {
-            explicit Captured(size_t bytes) : buffer(bytes) {}
-            DeviceBuffer buffer;
-            unsigned long long capture = 0;
-            cudaStream_t stream = nullptr;
-            std::shared_ptr<std::atomic<bool>> live;
-        };
-        void* capturedBuffer(unsigned long long capture, cudaGraph_t graph, cudaStream_t s,
-                             bool& fresh);
+        Captured& capturedBuffer(unsigned long long capture, cudaGraph_t graph, cudaStream_t s,
+                                 bool& fresh);
+        Kept* keptBuffer(unsigned long long stream, bool& fresh);
 
         DeviceBuffer buffer_;
         bool claimed_ = false;
-        cudaStream_t home_ = nullptr;
+        unsigned long long home_ = 0; // stream id (a handle may come back for another stream)
+        std::vector<std::unique_ptr<Kept>> kept_;
         std::vector<std::unique_ptr<Captured>> captured_;
     };
 

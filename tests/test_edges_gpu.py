@@ -143,29 +143,103 @@ def test_voxel_adjoint_same_footprints_at_size(cuda, oracle):
     assert rel_l2(fast, _apply(cuda, proj, y, True)) <= 5e-7
 
 
-@pytest.mark.parametrize("kind,vol,det", [("JOSEPH", (300, 280), [401]), ("JOSEPH", (120, 100), [150]),
-                                          ("SIDDON", (60, 50, 70), [90, 80]),
-                                          ("BLOB", (40, 50, 45), [60, 70]),
-                                          ("RAY_BLOB", (24, 20, 28), [40, 30])])
-def test_forwards_on_two_streams(cuda, oracle, kind, vol, det):
-    """The forwards' scratch is not shared between streams."""
+FORWARDS = [("JOSEPH", (300, 280), [401]), ("JOSEPH", (120, 100), [150]),
+            ("SIDDON", (60, 50, 70), [90, 80]), ("BLOB", (40, 50, 45), [60, 70]),
+            ("RAY_BLOB", (24, 20, 28), [40, 30])]
+
+
+@pytest.mark.parametrize("kind,vol,det", FORWARDS)
+@pytest.mark.parametrize("count", [2, 7])
+def test_forwards_on_several_streams(cuda, oracle, kind, vol, det, count):
+    """The forwards' scratch is not shared between streams: that of the first one, kept buffers of
+    others and, of the seven, temporary ones. Longer views and queues than a call takes to enqueue,
+    so that the streams overlap."""
     import elsa_b200
     torch = cuda
-    poses, det, x, _ = _problem(oracle, vol, 40, det)
-    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
-    xs = [torch.from_numpy(x).cuda() * (k + 1) for k in range(2)]
-    ref = [_apply(torch, proj, v.cpu().numpy(), False) for v in xs]
-    streams = [torch.cuda.Stream() for _ in range(2)]
-    outs = [[torch.empty(proj.range_size, device="cuda") for _ in range(4)] for _ in range(2)]
+    poses, det, x, _ = _problem(oracle, vol, 150, det)
+    make = lambda: elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    proj, other, repeats = make(), make(), 10
+    xs = [torch.from_numpy(x * np.float32(k + 1)).cuda() for k in range(count)]
+    ref = [_apply(torch, other, v.cpu().numpy(), False) for v in xs]
+    streams = [torch.cuda.Stream() for _ in range(count)]
+    outs = torch.zeros((count, repeats, proj.range_size), device="cuda")
+    # the streams' work waits for this product, so that all of it is enqueued by then
+    big = torch.zeros((8192, 8192), device="cuda")
     torch.cuda.synchronize()
-    for i in range(4):
+    for _ in range(4):
+        big = big @ big
+    start = torch.cuda.Event()
+    start.record()
+    for s in streams:
+        s.wait_event(start)
+    for i in range(repeats):
         for k, s in enumerate(streams):
             proj.apply_ptr(xs[k].data_ptr(), outs[k][i].data_ptr(), s.cuda_stream)
     torch.cuda.synchronize()
-    for k in range(2):
-        for o in outs[k]:
-            # (the voxel forward's atomics reorder its sums)
-            assert rel_l2(o.cpu().numpy(), ref[k]) <= (1e-6 if kind == "BLOB" else 0.0)
+    bound = 1e-6 if kind == "BLOB" else 0.0  # the voxel forward's atomics reorder its sums
+    for k in range(count):
+        for got in outs[k].cpu().numpy():
+            assert rel_l2(got, ref[k]) <= bound
+
+
+def test_forwards_on_streams_that_come_and_go(cuda, oracle):
+    """A program that makes a stream for every call keeps a bounded amount of scratch."""
+    import elsa_b200
+    torch = cuda
+    vol = (160, 150, 170)
+    poses, det, x, _ = _problem(oracle, vol, 4, [20, 20])
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_SIDDON, vol, det, poses)
+    ref = _apply(torch, proj, x, False)
+    d = torch.from_numpy(x).cuda()
+    y = torch.empty(proj.range_size, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for i in range(24):
+        s = torch.cuda.ExternalStream(_new_stream(torch))
+        y.zero_()
+        torch.cuda.synchronize()
+        proj.apply_ptr(d.data_ptr(), y.data_ptr(), s.cuda_stream)
+        if i % 3 == 0:
+            torch.cuda.synchronize()
+            assert np.array_equal(y.cpu().numpy(), ref)
+    torch.cuda.synchronize()
+    # two copies, four kept buffers of each, and one chunk of the device's pool
+    assert before - torch.cuda.mem_get_info()[0] <= 2 * 4 * 4 * x.size + (96 << 20)
+
+
+def _new_stream(torch):
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    s = ctypes.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(ctypes.byref(s), 1) == 0
+    return s.value
+
+
+@pytest.mark.parametrize("kind", ["SIDDON", "RAY_BLOB"])
+def test_forward_without_room_for_a_copy(cuda, oracle, kind):
+    """On a stream for which no scratch is left the volume itself is read."""
+    import elsa_b200
+    torch = cuda
+    vol = (300, 280, 320)
+    poses, det, x, _ = _problem(oracle, vol, 2, [24, 20])
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
+    ref = _apply(torch, proj, x, False)
+    d = torch.from_numpy(x).cuda()
+    y = torch.full((proj.range_size,), float("nan"), device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    full = []
+    try:
+        for piece in (1 << 30, 1 << 26, 1 << 24):
+            while torch.cuda.mem_get_info()[0] > (48 << 20) + piece:
+                full.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
+        proj.apply_ptr(d.data_ptr(), y.data_ptr(), s.cuda_stream)
+        torch.cuda.synchronize()
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    assert np.array_equal(y.cpu().numpy(), ref)
 
 
 @pytest.mark.parametrize("vol", [(20, 17, 23), (40, 33)])
@@ -322,11 +396,6 @@ def test_host_threads_on_one_stream(cuda, oracle, kind, vol, det, adjoint):
     for k in range(count):
         for got in outs[k].cpu().numpy():
             assert rel_l2(got, ref[k]) <= bound
-
-
-FORWARDS = [("JOSEPH", (300, 280), [401]), ("JOSEPH", (120, 100), [150]),
-            ("SIDDON", (60, 50, 70), [90, 80]), ("BLOB", (40, 50, 45), [60, 70]),
-            ("RAY_BLOB", (24, 20, 28), [40, 30])]
 
 
 @pytest.mark.parametrize("kind,vol,det", FORWARDS)
