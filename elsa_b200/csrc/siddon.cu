@@ -897,7 +897,6 @@ namespace elsa_b200
                         classSpacing_ = m;
                         break;
                     }
-                chooseLayouts();
                 const int bz = vol_.dim == 3 ? kSlab : 1;
                 nBricks_ = make_int3((vol_.n[0] + kSlab - 1) / kSlab,
                                      (vol_.n[1] + kSlab - 1) / kSlab, (vol_.n[2] + bz - 1) / bz);
@@ -914,6 +913,9 @@ namespace elsa_b200
                         need <= 0.5 * static_cast<double>(freeBytes))
                         setKnob(kKnobAdjointScatter, 0);
                 }
+                // last, since the volume itself serves where there is no room for the copies: they
+                // must not turn the adjoint to the scatter, nor take its partial volumes' memory
+                chooseLayouts();
                 ELSA_CUDA(cudaDeviceSynchronize());
             }
 

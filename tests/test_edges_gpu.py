@@ -22,6 +22,17 @@ def _apply(torch, proj, data, adjoint):
     return out.cpu().numpy()
 
 
+def _fill_memory(torch, leave):
+    """Tensors that leave `leave` bytes (to 16 MiB) of the device's memory free."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    full = []
+    for piece in (1 << 30, 1 << 26, 1 << 24):
+        while torch.cuda.mem_get_info()[0] > leave + piece:
+            full.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
+    return full
+
+
 def _problem(oracle, vol, views, det, arc=360, seed=3):
     n = max(vol)
     poses, det = oracle.circle_trajectory(vol, views, arc, 5.0 * n, 1.5 * n, det)
@@ -227,13 +238,8 @@ def test_forward_without_room_for_a_copy(cuda, oracle, kind):
     d = torch.from_numpy(x).cuda()
     y = torch.full((proj.range_size,), float("nan"), device="cuda")
     s = torch.cuda.Stream()
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    full = []
+    full = _fill_memory(torch, 48 << 20)
     try:
-        for piece in (1 << 30, 1 << 26, 1 << 24):
-            while torch.cuda.mem_get_info()[0] > (48 << 20) + piece:
-                full.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
         proj.apply_ptr(d.data_ptr(), y.data_ptr(), s.cuda_stream)
         torch.cuda.synchronize()
     finally:
@@ -462,3 +468,35 @@ def test_captures_reuse_scratch(cuda, oracle):
     for _ in range(20):
         capture()
     assert free - torch.cuda.mem_get_info()[0] <= 4 * 2 * 4 * x.size  # of 20 captures' two copies
+
+
+def test_siddon_copies_leave_the_adjoint_its_tables(cuda):
+    """Where the adjoint's tables just fit its rule (half of what is free beside the rays), the
+    forward's volume copy does not turn it to the scatter."""
+    import elsa_b200
+    torch = cuda
+    n, pixels = 512, 1000
+    one = [1.0] * 3
+    pose = elsa_b200.pose_3d(5.0 * n, 1.5 * n, one, [0.5 * n] * 3, one,
+                             [0.5 * pixels, 0.5 * pixels, 0.0], 0.5 * np.pi)  # drives along x
+    make = lambda: elsa_b200.Projector(elsa_b200.PROJECTOR_SIDDON, (n,) * 3,
+                                       [pixels, pixels, 1], pose)
+    torch.cuda.synchronize()
+    x = torch.rand(n ** 3, device="cuda")
+    y = torch.empty(pixels * pixels, device="cuda")
+    out = []
+    for limited in (False, True):
+        rays = pixels * pixels
+        tables, setup, copy = 20 * rays * (n // 16 + 3), 128 * rays, 4 * n ** 3
+        full = _fill_memory(torch, 2 * tables + setup + copy // 2) if limited else []
+        try:
+            proj = make()
+            assert proj.knob(elsa_b200.KNOB_ADJOINT_SCATTER) == 0
+            proj.apply_ptr(x.data_ptr(), y.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+        finally:
+            del full
+        out.append(y.cpu().numpy())
+        proj.close()
+        torch.cuda.empty_cache()
+    assert np.array_equal(*out)
