@@ -126,21 +126,70 @@ namespace elsa_b200
             int64_t stride[3][3];
         };
 
-        // One thread per ray, the reference's visits and float operations in order. Bound by issue
-        // (about 25 instructions per visit) once neighbouring lanes read neighbouring words: with
+        // 2D: one thread per ray on the image itself. A ray is a few hundred visits and a launch a few
+        // warps per SM, so the time is the chain of a visit: the predicated form of the 3D kernel
+        // below is slower here (256 x 231 / 300 views / 365 pixels: 81 us beside 5 of the image's copy,
+        // this one 65), and a transposed image buys nothing while it stays in L1 and L2 (1000 x 900 /
+        // 30 views: 320 us with it, 314 without).
+        __global__ void __launch_bounds__(kMaxForwardThreads)
+            siddonForward2dKernel(const SiddonRay* __restrict__ rays, int64_t nrays,
+                                  const float* __restrict__ x, VolumeShape vol, int binary,
+                                  float* __restrict__ y)
+        {
+            // binary: BinaryMethod (projectors/BinaryMethod.cpp:66-111), weight 1 per visit
+            const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+            if (r >= nrays)
+                return;
+            const SiddonRay R = rays[r];
+            float acc = 0.0f;
+            if (R.meta & kActive) {
+                int c0, c1, c2;
+                entryVoxel(R.meta & 3, R.kFirst, R.cur[0], R.cur[1], c0, c1, c2);
+                const int s0 = axisStep(R.meta, 0), s1 = axisStep(R.meta, 1);
+                const int nx = vol.n[0], ny = vol.n[1];
+                const int64_t sy = nx;
+                int64_t idx = c0 + sy * c1;
+                float T0 = R.T[0], T1 = R.T[1];
+                float tExit = 0.0f;
+                const int maxVisits = nx + ny + 3;
+                for (int it = 0; it < maxVisits; ++it) {
+                    const float tEntry = tExit;
+                    bool m0, m1, m2;
+                    tExit = nextCrossing<2>(T0, T1, 0.0f, m0, m1, m2);
+                    if (m0) {
+                        c0 += s0;
+                        T0 = __fadd_rn(T0, R.tDelta[0]);
+                    }
+                    if (m1) {
+                        c1 += s1;
+                        T1 = __fadd_rn(T1, R.tDelta[1]);
+                    }
+                    const float w = binary ? 1.0f : __fsub_rn(tExit, tEntry);
+                    acc = __fadd_rn(acc, __fmul_rn(__ldg(x + idx), w));
+                    if (static_cast<unsigned>(c0) >= static_cast<unsigned>(nx) ||
+                        static_cast<unsigned>(c1) >= static_cast<unsigned>(ny))
+                        break;
+                    idx += (m0 ? s0 : 0) + (m1 ? s1 * sy : 0);
+                }
+            }
+            y[r] = acc;
+        }
+
+        // 3D: one thread per ray, the reference's visits and float operations in order. Bound by issue
+        // (29 instructions per visit) once neighbouring lanes read neighbouring words: with
         // every ray on the x-fastest volume, a warp whose rays drive along x read 32 sectors per
         // visit and the load pipe took the time (171 x 200 x 149 voxels, 240 views of
         // 250 x 231: 3.62 ms, now 2.69). The bounds test counts the steps left along each axis, so
         // a visit updates one word offset instead of three voxel indices and a 64-bit one. Offset:
         // unsigned below 2^32 words, else int64_t.
-        template <int DIM, typename Offset>
+        template <typename Offset>
         __global__ void __launch_bounds__(kMaxForwardThreads)
             siddonForwardKernel(const SiddonRay* __restrict__ rays, int64_t nrays,
                                 const __grid_constant__ SiddonLayouts layouts, VolumeShape vol,
                                 int binary,
                                 float* __restrict__ y)
         {
-            // binary: BinaryMethod (projectors/BinaryMethod.cpp:66-111), weight 1 per visit
+            // binary: weight 1 per visit, as above
             const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
             if (r >= nrays)
                 return;
@@ -155,25 +204,24 @@ namespace elsa_b200
                 const float* base = layouts.base[g];
                 const Offset e0 = static_cast<Offset>(layouts.stride[g][0]),
                              e1 = static_cast<Offset>(layouts.stride[g][1]),
-                             e2 = DIM == 3 ? static_cast<Offset>(layouts.stride[g][2]) : 0;
-                Offset idx = c0 * e0 + c1 * e1 + (DIM == 3 ? c2 * e2 : 0);
+                             e2 = static_cast<Offset>(layouts.stride[g][2]);
+                Offset idx = c0 * e0 + c1 * e1 + c2 * e2;
                 const Offset i0 = s0 * e0, i1 = s1 * e1, i2 = s2 * e2;
                 // steps left before the ray leaves the volume (the entry voxel is inside)
                 int left0 = s0 > 0 ? vol.n[0] - 1 - c0 : c0;
                 int left1 = s1 > 0 ? vol.n[1] - 1 - c1 : c1;
-                int left2 = DIM == 3 ? (s2 > 0 ? vol.n[2] - 1 - c2 : c2) : 0;
+                int left2 = s2 > 0 ? vol.n[2] - 1 - c2 : c2;
                 const int k0 = s0 != 0, k1 = s1 != 0, k2 = s2 != 0;
                 float T0 = R.T[0], T1 = R.T[1], T2 = R.T[2];
                 float tExit = 0.0f;
-                const int maxVisits = vol.n[0] + vol.n[1] + (DIM == 3 ? vol.n[2] : 0) + 3;
+                const int maxVisits = vol.n[0] + vol.n[1] + vol.n[2] + 3;
                 for (int it = 0; it < maxVisits; ++it) {
                     const float v = __ldg(base + idx);
                     const float tEntry = tExit;
-                    tExit = DIM == 3 ? fminf(T0, fminf(T1, T2)) : fminf(T0, T1);
+                    tExit = fminf(T0, fminf(T1, T2));
                     crossIf(tExit, T0, R.tDelta[0], idx, i0, left0, k0);
                     crossIf(tExit, T1, R.tDelta[1], idx, i1, left1, k1);
-                    if (DIM == 3)
-                        crossIf(tExit, T2, R.tDelta[2], idx, i2, left2, k2);
+                    crossIf(tExit, T2, R.tDelta[2], idx, i2, left2, k2);
                     const float w = binary ? 1.0f : __fsub_rn(tExit, tEntry);
                     acc = __fadd_rn(acc, __fmul_rn(v, w));
                     if ((left0 | left1 | left2) < 0)
@@ -915,40 +963,48 @@ namespace elsa_b200
                 }
                 // last, since the volume itself serves where there is no room for the copies: they
                 // must not turn the adjoint to the scatter, nor take its partial volumes' memory
-                chooseLayouts();
+                if (vol_.dim == 3)
+                    chooseLayouts();
                 ELSA_CUDA(cudaDeviceSynchronize());
             }
 
-            // The axis that is contiguous in the volume each driving axis is read from, and the
-            // copies' buffers (for the driving axes that occur).
+            // 3D: the axis that is contiguous in the volume each driving axis is read from, and the
+            // copies' buffers (for the driving axes that occur). A copy costs about 8 us and 5 ps per
+            // voxel on every call; per visit of a view that reads it, it saves about 0.9 ps, and 3
+            // where the volume is larger than L2. It is made where that is 1.5 times the cost.
+            // Copy / none: 128^3 / 192^2, 30 views 199 / 221 us, 8 views 88 / 78, 8 views that all
+            // drive along x 70 / 84; 64^3 / 90 views 87 / 95; 32^3 / 40 views 18.5 / 13.3; 500^3 /
+            // 8 views, 600^2 2732 / 3482, 200^2 810 / 381.
             void chooseLayouts()
             {
                 std::vector<unsigned> axes(static_cast<size_t>(det_.np));
                 ELSA_CUDA(cudaMemcpy(axes.data(), viewAxes_->as<unsigned>(),
                                      sizeof(unsigned) * axes.size(), cudaMemcpyDeviceToHost));
-                unsigned present = 0;
-                for (unsigned a : axes)
-                    present |= a;
-                if (vol_.dim == 3) {
-                    std::vector<float> hp(poses_.size() * kPoseFloats);
-                    std::memcpy(hp.data(), poses_.data(), sizeof(float) * hp.size());
-                    fast_ = fastAxes(hp, det_);
-                } else {
-                    fast_ = {1, 0, 0};
-                }
-                for (int g = 0; g < vol_.dim; ++g) {
-                    const int f = fast_[g];
-                    if (!((present >> g) & 1u)) {
-                        fast_[g] = 0;
-                    } else if (f != 0 && !copies_[f]) {
-                        try {
-                            copies_[f] = std::make_unique<StreamScratch>(
-                                sizeof(float) * static_cast<size_t>(domainSize_));
-                        } catch (const Error&) { // no room: the volume itself serves
-                            cudaGetLastError();
-                            fast_[g] = 0;
-                        }
+                std::vector<float> hp(poses_.size() * kPoseFloats);
+                std::memcpy(hp.data(), poses_.data(), sizeof(float) * hp.size());
+                const std::array<int, 3> fast = fastAxes(hp, det_);
+                constexpr double kL2Bytes = 1e8; // (126 MB, shared with the sinogram and the rays)
+                const double perVoxel = 4.0 * domainSize_ > kL2Bytes ? 2.8 : 8.3;
+                const double least = 1.3e7 + perVoxel * static_cast<double>(domainSize_);
+                for (int f = 1; f < 3; ++f) {
+                    unsigned readers = 0; // driving axes that would read this copy
+                    for (int g = 0; g < 3; ++g)
+                        if (fast[g] == f)
+                            readers |= 1u << g;
+                    const auto views = std::count_if(axes.begin(), axes.end(),
+                                                     [&](unsigned a) { return a & readers; });
+                    if (static_cast<double>(visits_) * views <= least * det_.np)
+                        continue;
+                    try {
+                        copies_[f] = std::make_unique<StreamScratch>(
+                            sizeof(float) * static_cast<size_t>(domainSize_));
+                    } catch (const Error&) { // no room: the volume itself serves
+                        cudaGetLastError();
+                        continue;
                     }
+                    for (int g = 0; g < 3; ++g)
+                        if (fast[g] == f)
+                            fast_[g] = f;
                 }
             }
 
@@ -957,6 +1013,12 @@ namespace elsa_b200
                 const int64_t nrays = rangeSize_;
                 const unsigned blocks =
                     static_cast<unsigned>((nrays + forwardThreads_ - 1) / forwardThreads_);
+                if (vol_.dim == 2) {
+                    siddonForward2dKernel<<<blocks, forwardThreads_, 0, s>>>(
+                        rays_->as<SiddonRay>(), nrays, x, vol_, binary_, y);
+                    ELSA_LAUNCH_CHECK("siddonForward2dKernel");
+                    return;
+                }
                 SiddonLayouts layouts;
                 const int64_t plane = static_cast<int64_t>(vol_.n[0]) * vol_.n[1];
                 for (int g = 0; g < 3; ++g) {
@@ -965,7 +1027,7 @@ namespace elsa_b200
                     layouts.stride[g][2] = plane;
                 }
                 std::unique_ptr<StreamScratch::Lease> copies[3];
-                for (int f = 1; f < vol_.dim; ++f) {
+                for (int f = 1; f < 3; ++f) {
                     if (!copies_[f])
                         continue;
                     copies[f] = std::make_unique<StreamScratch::Lease>(*copies_[f], s, true);
@@ -976,17 +1038,14 @@ namespace elsa_b200
                     int64_t stride[3];
                     stride[f] = 1, stride[0] = nf, stride[3 - f] = nf * vol_.n[0];
                     launchLayoutCopy(x, vol_, f, stride, copies[f]->as<float>(), s);
-                    for (int g = 0; g < vol_.dim; ++g)
+                    for (int g = 0; g < 3; ++g)
                         if (fast_[g] == f) {
                             layouts.base[g] = copies[f]->as<float>();
                             std::copy(stride, stride + 3, layouts.stride[g]);
                         }
                 }
-                const bool narrow = domainSize_ < (int64_t(1) << 32);
-                auto* k = vol_.dim == 3 ? (narrow ? siddonForwardKernel<3, unsigned>
-                                                  : siddonForwardKernel<3, int64_t>)
-                                        : (narrow ? siddonForwardKernel<2, unsigned>
-                                                  : siddonForwardKernel<2, int64_t>);
+                auto* k = domainSize_ < (int64_t(1) << 32) ? siddonForwardKernel<unsigned>
+                                                           : siddonForwardKernel<int64_t>;
                 k<<<blocks, forwardThreads_, 0, s>>>(rays_->as<SiddonRay>(), nrays, layouts, vol_,
                                                      binary_, y);
                 ELSA_LAUNCH_CHECK("siddonForwardKernel");
