@@ -111,6 +111,17 @@ def test_ray_lut_layouts(cuda, oracle, vol, views, det, kind):
     assert rel_l2(_apply(cuda, proj, y, True), ref) <= PARITY
 
 
+VOXEL_KINDS = [("blob", (2.0, 10.83, 2)), ("bspline", (3,)), ("phase_blob", (2.0, 10.83, 2)),
+               ("phase_bspline", (3,))]
+VOXEL_CODES = {"blob": 2, "bspline": 3, "phase_blob": 4, "phase_bspline": 5}
+
+
+def _voxel_reference(oracle, kind, params, dim):
+    if kind.endswith("blob"):
+        return oracle.voxel_lut(kind, dim, *params)
+    return oracle.voxel_lut(kind, dim, order=params[0])
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("kind,params", [
     ("blob", (2.0, 10.83, 2)), ("blob", (0.55, 10.83, 2)), ("blob", (3.7, 8.0, 1)),
@@ -141,6 +152,43 @@ def test_voxel_footprints(cuda, oracle, vol, views, det, kind, params, mode):
     assert np.array_equal(exact, np.asarray(oracle.voxel_project(True, y, *args), np.float32))
     # phase-contrast sums cancel: weights of both signs, relative to their magnitude
     assert rel_l2(fast, exact) <= (PARITY if kind.startswith("phase") else 2e-6)
+
+
+# voxels times poses above the small problems', which have a forward of their own
+LATTICE = [((50, 60, 49), 41, [70, 61]), ((200, 37), 90, [250]), ((60, 75), 110, [80]),
+           ((20, 400), 60, [560])]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kind,params", [
+    ("blob", (2.0, 10.83, 2)), ("blob", (3.7, 8.0, 1)), ("blob", (0.55, 10.83, 2)),
+    ("bspline", (5,)), ("phase_blob", (3.1, 10.83, 2))])
+@pytest.mark.parametrize("vol,views,det", LATTICE)
+def test_voxel_lattice(cuda, oracle, vol, views, det, kind, params, mode):
+    """The forward of larger problems: lattices of several tiles and rows of 32, 16, 8 and 4
+    voxels, patches clipped by the detector."""
+    import elsa_b200
+    poses, det, x, _ = _problem(oracle, vol, views, det)
+    x[::3] = 0.0
+    proj = elsa_b200.Projector(VOXEL_CODES[kind], vol, det, poses,
+                               tuple(map(float, params)) + (mode,))
+    ref = oracle.voxel_project(False, x, vol, det, poses,
+                               *_voxel_reference(oracle, kind, params, len(vol)), mode)
+    for _ in range(2):  # the second one starts from what the first left in its counter
+        assert rel_l2(_apply(cuda, proj, x, False), ref) <= PARITY
+
+
+@pytest.mark.parametrize("radius", [6.0, 9.0])
+@pytest.mark.parametrize("vol,views,det", LATTICE)
+def test_voxel_lattice_of_wide_footprints(cuda, oracle, vol, views, det, radius):
+    """Lattices that do not fit their patch or overlap (shared atomics), against the adjoint of the
+    same weights: <A x, y> = <x, A^T y>."""
+    import elsa_b200
+    poses, det, x, y = _problem(oracle, vol, views, det)
+    proj = elsa_b200.Projector(elsa_b200.PROJECTOR_BLOB, vol, det, poses, (radius, 10.83, 2.0, 1.0))
+    ax = _apply(cuda, proj, x, False).astype(np.float64)
+    aty = _apply(cuda, proj, y, True).astype(np.float64)
+    assert abs(ax @ y - x @ aty) <= 1e-6 * (ax @ y)
 
 
 def test_voxel_adjoint_same_footprints_at_size(cuda, oracle):
@@ -316,25 +364,15 @@ def test_batched_solve_with_an_operator_that_meets_nothing(cuda, oracle):
     assert not batch.squared_residuals(s)[1] > 0.0  # 0 / 0 afterwards, as in a solve of its own
 
 
-VOXEL_KINDS = [("blob", (2.0, 10.83, 2)), ("bspline", (3,)), ("phase_blob", (2.0, 10.83, 2)),
-               ("phase_bspline", (3,))]
-VOXEL_CODES = {"blob": 2, "bspline": 3, "phase_blob": 4, "phase_bspline": 5}
-
-
-def _voxel_reference(oracle, kind, params, dim):
-    if kind.endswith("blob"):
-        return oracle.voxel_lut(kind, dim, *params)
-    return oracle.voxel_lut(kind, dim, order=params[0])
-
-
 @pytest.mark.parametrize("kind,params", VOXEL_KINDS)
-@pytest.mark.parametrize("s2c,c2d", [(-100.0, 300.0), (-40.0, 90.0), (-90.0, 30.0), (6.0, 90.0)])
-@pytest.mark.parametrize("vol,det", [((13, 21, 9), [17, 12]), ((30, 23), [41])])
-def test_voxel_source_in_front_or_inside(cuda, oracle, vol, det, s2c, c2d, kind, params):
+@pytest.mark.parametrize("s2c,c2d", [(-100.0, 300.0), (-40.0, 90.0), (-90.0, 30.0), (6.0, 20.0)])
+@pytest.mark.parametrize("vol,views,det", [((13, 21, 9), 5, [17, 12]), ((30, 23), 5, [41]),
+                                           ((60, 50), 160, [70]), ((46, 48, 50), 55, [60, 62])])
+def test_voxel_source_in_front_or_inside(cuda, oracle, vol, views, det, s2c, c2d, kind, params):
     """A volume behind the source projects as well (quotients of two negative numbers), also with
     a negative source-detector distance, and around a source inside the volume."""
     import elsa_b200
-    poses, det = elsa_b200.circle_trajectory(vol, 5, 300.0, s2c, c2d, det)
+    poses, det = elsa_b200.circle_trajectory(vol, views, 300.0, s2c, c2d, det)
     rng = np.random.default_rng(4)
     x = rng.uniform(0, 1, int(np.prod(vol))).astype(np.float32)
     y = rng.uniform(0, 1, int(np.prod(det))).astype(np.float32)
@@ -345,7 +383,8 @@ def test_voxel_source_in_front_or_inside(cuda, oracle, vol, det, s2c, c2d, kind,
     assert rel_l2(_apply(cuda, proj, y, True), oracle.voxel_project(True, y, *args)) <= PARITY
 
 
-@pytest.mark.parametrize("vol,det", [((13, 21, 9), [17, 12]), ((30, 23), [41])])
+@pytest.mark.parametrize("vol,det", [((13, 21, 9), [17, 12]), ((30, 23), [41]),
+                                     ((400, 390), [500]), ((130, 128, 126), [170, 166])])
 def test_voxel_pose_of_nan(cuda, oracle, vol, det):
     """A pose that is not a number spoils its own view and no other."""
     import elsa_b200
@@ -373,7 +412,7 @@ def test_host_threads_on_one_stream(cuda, oracle, kind, vol, det, adjoint):
     import threading
     import elsa_b200
     torch = cuda
-    poses, det, x, y = _problem(oracle, vol, 100 if kind == "SIDDON" else 12, det)
+    poses, det, x, y = _problem(oracle, vol, 100 if kind in ("SIDDON", "BLOB") else 12, det)
     proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
     base = y if adjoint else x
     count, repeats = 4, 60
