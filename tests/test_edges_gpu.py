@@ -128,7 +128,7 @@ def _voxel_reference(oracle, kind, params, dim):
     ("blob", (9.0, 10.83, 2)), ("blob", (1.3, 2.0, 0)), ("bspline", (0,)), ("bspline", (5,)),
     ("phase_blob", (3.1, 10.83, 2)), ("phase_bspline", (3,))])
 @pytest.mark.parametrize("vol,views,det", [((13, 21, 9), 7, [17, 12]), ((50, 6, 49), 5, [70, 31]),
-                                           ((200, 7), 6, [90])])
+                                           ((200, 7), 6, [90]), ((60, 41), 11, [70])])
 def test_voxel_footprints(cuda, oracle, vol, views, det, kind, params, mode):
     """Footprints of one pixel to more than six columns, lattices that overlap (shared atomics),
     patches that do not fit, tables that do not end in 0, voxels projected off the detector. The
