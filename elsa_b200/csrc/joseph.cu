@@ -17,7 +17,7 @@
 // accumulates from there.
 //
 // Forward: joseph_tma.cu in 3D; in 2D a warp takes 32 neighbouring rays through a checkpoint slab,
-// reading zero-padded copies of the image's rows and columns.
+// reading zero-padded copies of the image's rows and columns (the image itself for small problems).
 //
 // Adjoint (default): atomic-free and deterministic. Each warp owns one brick (2D: tile) of the
 // volume in shared memory for a chunk of the views. For every view it visits the rays of the
@@ -636,9 +636,33 @@ namespace elsa_b200
             return acc;
         }
 
+        // The same samples from the image itself: line k's pixel i at q + i * tapStep.
+        __device__ __forceinline__ float imageSamples(const float* q, int lineStep, int tapStep,
+                                                      float p, float s, int count, int n)
+        {
+            float acc = 0.0f;
+            for (int j = 0; j < count; ++j) {
+                int i;
+                const float h = __fsub_rn(p, 0.5f);
+                const float cw = __fsub_rn(h, floorSmall(h, i));
+                const bool in0 = static_cast<unsigned>(i) < static_cast<unsigned>(n);
+                const bool in1 = static_cast<unsigned>(i + 1) < static_cast<unsigned>(n);
+                const float v0 = in0 ? __ldg(q + i * tapStep) : 0.0f;
+                const float v1 = in1 ? __ldg(q + (i + 1) * tapStep) : 0.0f;
+                acc = __fmaf_rn(__fsub_rn(1.0f, cw), v0, acc);
+                acc = __fmaf_rn(cw, v1, acc);
+                p = __fadd_rn(p, s);
+                q += lineStep;
+            }
+            return acc;
+        }
+
         // blockDim.x = 32 lanes (neighbouring rays of one view), blockDim.y = warps: `groups` groups
         // of warps, one view each, the warps of a group dividing its slabs. A block's views follow
-        // one another, so its groups read nearly the same lines from L1.
+        // one another, so its groups read nearly the same lines from L1. Padded: from rows and
+        // columns; otherwise from the image (rows), for images so small that the launch that pads them
+        // is not repaid.
+        template <bool Padded>
         __global__ void __launch_bounds__(kMaxForwardThreads)
             josephForward2dKernel(const JosephRay* __restrict__ rays,
                                   const float2* __restrict__ checkpoints, int64_t nrays,
@@ -661,7 +685,7 @@ namespace elsa_b200
             const int dir = (R.meta & 4) ? -1 : 1;
             const int n = g == 0 ? vol.n[1] : vol.n[0], ng = g == 0 ? vol.n[0] : vol.n[1];
             const int pitch = linePitch(n);
-            const float* lines = (g == 0 ? columns : rows) + kLinePad;
+            const float* lines = (g == 0 ? columns : rows) + kLinePad; // (Padded)
             float acc = 0.0f;
             for (int slab = member; slab < nSlabs; slab += perGroup) {
                 int jLo, jHi;
@@ -674,6 +698,12 @@ namespace elsa_b200
                     pos = __fadd_rn(pos, R.sa);
                 if (dir > 0)
                     count = min(count, ng - k);
+                if (!Padded) {
+                    const int lineStep = g == 0 ? 1 : vol.n[0], tapStep = g == 0 ? vol.n[0] : 1;
+                    acc += imageSamples(rows + k * lineStep, dir * lineStep, tapStep, pos, R.sa,
+                                        count, n);
+                    continue;
+                }
                 // positions are monotone along the ray; a sample's line words are within the
                 // padding unless the positions leave the image by several voxels
                 const float end = pos + R.sa * static_cast<float>(count);
@@ -1218,8 +1248,14 @@ namespace elsa_b200
         // blocks; their rays start and end in more tiles).
         using Adjoint2dLarge = Adjoint2dConfig<64, 4>;
         using Adjoint2dSmall = Adjoint2dConfig<32, 8>;
-                constexpr int kSmallImage = 256 * 256; // pixels (512^2 adjoint: 0.504 ms with tiles of 32,
-                                               // 0.514 of 64, which need half the checkpoints)
+        // pixels up to which the tiles are the small ones (for 512^2 they are as fast, 0.504 ms against
+        // 0.514, but need twice the checkpoints)
+        constexpr int kSmallImage = 256 * 256;
+        // Pixels, and pixels times views, up to which the forward reads the image itself. Padded /
+        // direct in us, 1.45 pixels per column: 32^2 / 40 views 14.3 / 8.6; 80^2 / 180 (1.15e6)
+        // 18.5 / 10.6; 96^2 / 180 (1.7e6) 20.5 / 25.2; 128^2 / 40 14.4 / 12.3, / 180 15.1 / 18.9.
+        constexpr int kDirectImage = 128 * 128;
+        constexpr int64_t kDirectWork = 1200000;
 
         class JosephProjector final : public Projector
         {
@@ -1317,6 +1353,8 @@ namespace elsa_b200
                 const int tile = domainSize_ <= kSmallImage ? 32 : 64;
                 brick_ = make_int3(tile, tile, 1);
                 buildCheckpoints(tile);
+                if (domainSize_ <= kDirectImage && domainSize_ * det_.np <= kDirectWork)
+                    return;
                 lines_ = std::make_unique<StreamScratch>(
                     sizeof(float) * (rowWords() + static_cast<size_t>(vol_.n[0]) *
                                                       linePitch(vol_.n[1])));
@@ -1461,15 +1499,19 @@ namespace elsa_b200
 
             void forward2d(const float* x, float* y, cudaStream_t s)
             {
-                const StreamScratch::Lease lines(*lines_, s);
-                if (lines.fresh()) // the padding
-                    ELSA_CUDA(cudaMemsetAsync(lines.as<void>(), 0, lines_->bytes(), s));
-                float* rows = lines.as<float>();
-                float* columns = rows + rowWords();
-                const dim3 blocks((vol_.n[0] + 31) / 32, (vol_.n[1] + 31) / 32);
-                padLinesKernel<<<blocks, dim3(32, 8), 0, s>>>(
-                    x, vol_.n[0], vol_.n[1], rows, columns);
-                ELSA_LAUNCH_CHECK("padLinesKernel");
+                std::unique_ptr<StreamScratch::Lease> lines;
+                const float *rows = x, *columns = nullptr; // (small images: the image itself)
+                if (lines_) {
+                    lines = std::make_unique<StreamScratch::Lease>(*lines_, s);
+                    if (lines->fresh()) // the padding
+                        ELSA_CUDA(cudaMemsetAsync(lines->as<void>(), 0, lines_->bytes(), s));
+                    float* padded = lines->as<float>();
+                    const dim3 blocks((vol_.n[0] + 31) / 32, (vol_.n[1] + 31) / 32);
+                    padLinesKernel<<<blocks, dim3(32, 8), 0, s>>>(x, vol_.n[0], vol_.n[1], padded,
+                                                                  padded + rowWords());
+                    ELSA_LAUNCH_CHECK("padLinesKernel");
+                    rows = padded, columns = padded + rowWords();
+                }
                 const int depth = 1 << cpdShift_;
                 const int slabs = (std::max(vol_.n[0], vol_.n[1]) + depth - 1) / depth;
                 const int segments = (det_.nu + 31) / 32;
@@ -1482,9 +1524,10 @@ namespace elsa_b200
                 const int groups = warps / perGroup;
                 const int64_t grid =
                     static_cast<int64_t>(segments) * ((det_.np + groups - 1) / groups);
-                josephForward2dKernel<<<static_cast<unsigned>(grid), dim3(32, groups * perGroup), 0,
-                                        s>>>(dRays_, dCheckpoints_, rangeSize_, vol_, det_, depth,
-                                             slabs, groups, segments, rows, columns, y);
+                auto* k = lines_ ? josephForward2dKernel<true> : josephForward2dKernel<false>;
+                k<<<static_cast<unsigned>(grid), dim3(32, groups * perGroup), 0, s>>>(
+                    dRays_, dCheckpoints_, rangeSize_, vol_, det_, depth, slabs, groups, segments,
+                    rows, columns, y);
                 ELSA_LAUNCH_CHECK("josephForward2dKernel");
             }
 
@@ -1808,7 +1851,7 @@ namespace elsa_b200
                 case 4: // parts per million of detector tiles on the gather fallback
                     return tma_ ? static_cast<int64_t>(tma_->fallbackFraction() * 1e6) : -1;
                 case 6: // kernel launches per forward call
-                    return tma_ ? tma_->launchesPerForward() : 2;
+                    return tma_ ? tma_->launchesPerForward() : (lines_ ? 2 : 1);
                 case 7: // kernel launches per adjoint call (3D: one per axis grid; with
                         // several partial volumes: + the chunk sum)
                     if (fast_ || scatter_)

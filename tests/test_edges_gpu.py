@@ -44,10 +44,11 @@ def _problem(oracle, vol, views, det, arc=360, seed=3):
 
 @pytest.mark.parametrize("vol,views,det", [
     ((1, 1), 3, [3]), ((31, 33), 5, [31]), ((32, 32), 7, [33]), ((65, 40), 9, [64]),
-    ((127, 1), 4, [140]), ((256, 257), 6, [321]), ((300, 290), 11, [401]), ((1, 70), 8, [97])])
+    ((127, 1), 4, [140]), ((256, 257), 6, [321]), ((300, 290), 11, [401]), ((1, 70), 8, [97]),
+    ((128, 128), 73, [182]), ((128, 128), 74, [182]), ((33, 31), 1200, [45])])
 def test_joseph_2d_tiles(cuda, oracle, vol, views, det):
-    """Tiles of 32 and 64 pixels, remainders, one-pixel edges; views around 45 degrees mix both
-    driving axes."""
+    """Tiles of 32 and 64 pixels, remainders, one-pixel edges, from the image and from its padded
+    lines; views around 45 degrees mix both driving axes."""
     import elsa_b200
     poses, det, x, y = _problem(oracle, vol, views, det)
     proj = elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, poses)
@@ -62,12 +63,14 @@ def test_joseph_2d_tiles(cuda, oracle, vol, views, det):
     assert rel_l2(_apply(cuda, proj, y, True), ref) <= PARITY
 
 
-def test_joseph_2d_non_finite(cuda, oracle):
-    """An infinity reaches exactly the pixels whose rays meet it, as in the oracle."""
+@pytest.mark.parametrize("vol,views,det", [((40, 37), 6, [50]), ((140, 137), 9, [200]),
+                                           ((100, 60), 210, [150])])
+def test_joseph_2d_non_finite(cuda, oracle, vol, views, det):
+    """An infinity reaches exactly the pixels whose rays meet it, as in the oracle, from the image
+    and from its padded lines."""
     import elsa_b200
-    vol = (40, 37)
-    poses, det, x, _ = _problem(oracle, vol, 6, [50])
-    x[20 + 40 * 11] = np.inf
+    poses, det, x, _ = _problem(oracle, vol, views, det)
+    x[20 + vol[0] * 11] = np.inf
     proj = elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, poses)
     got = _apply(cuda, proj, x, False)
     ref = np.asarray(oracle.joseph(x, vol, det, poses))
@@ -412,7 +415,7 @@ def test_host_threads_on_one_stream(cuda, oracle, kind, vol, det, adjoint):
     import threading
     import elsa_b200
     torch = cuda
-    poses, det, x, y = _problem(oracle, vol, 100 if kind in ("SIDDON", "BLOB") else 12, det)
+    poses, det, x, y = _problem(oracle, vol, 110, det)
     proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, poses)
     base = y if adjoint else x
     count, repeats = 4, 60
