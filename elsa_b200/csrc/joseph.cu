@@ -1297,10 +1297,11 @@ namespace elsa_b200
                         classSpacing_ = m;
                         break;
                     }
+                if (fast_)
+                    buildFastAdjoint();
                 if (vol_.dim == 2)
                     buildForward2d();
                 if (fast_) {
-                    buildFastAdjoint();
                     if (vol_.dim == 3) {
                         std::vector<float> hp(poses_.size() * kPoseFloats);
                         std::memcpy(hp.data(), poses_.data(), sizeof(float) * hp.size());
@@ -1347,18 +1348,43 @@ namespace elsa_b200
                 curved_.release(); // rays and windows are built
             }
 
-            // 2D: checkpoints, one slab per tile of the adjoint, and the padded image copies.
+            // 2D: checkpoints, one slab per tile of the matched adjoint, and the padded image copies.
             void buildForward2d()
             {
-                const int tile = domainSize_ <= kSmallImage ? 32 : 64;
+                if (domainSize_ > kDirectImage || domainSize_ * det_.np > kDirectWork) {
+                    lines_ = std::make_unique<StreamScratch>(
+                        sizeof(float) * (rowWords() + static_cast<size_t>(vol_.n[0]) *
+                                                          linePitch(vol_.n[1])));
+                    ELSA_CUDA(cudaMemset(lines_->initial(), 0, lines_->bytes()));
+                }
+                const int maxDim = std::max(vol_.n[0], vol_.n[1]);
+                auto fits = [&](int cpd) { // the table in an eighth of the device's memory, as in 3D
+                    const double bytes =
+                        8.0 * static_cast<double>(rangeSize_) * (maxDim / cpd + 3);
+                    if (bytes < 1e9)
+                        return true; // (asking takes half a millisecond)
+                    size_t freeBytes = 0, totalBytes = 0;
+                    ELSA_CUDA(cudaMemGetInfo(&freeBytes, &totalBytes));
+                    return bytes <= static_cast<double>(totalBytes) / 8.0;
+                };
+                const int tile = domainSize_ <= kSmallImage && fits(32) ? 32 : 64;
                 brick_ = make_int3(tile, tile, 1);
-                buildCheckpoints(tile);
-                if (domainSize_ <= kDirectImage && domainSize_ * det_.np <= kDirectWork)
-                    return;
-                lines_ = std::make_unique<StreamScratch>(
-                    sizeof(float) * (rowWords() + static_cast<size_t>(vol_.n[0]) *
-                                                      linePitch(vol_.n[1])));
-                ELSA_CUDA(cudaMemset(lines_->initial(), 0, lines_->bytes()));
+                // The `fast` adjoint has no checkpoints: its forward takes deeper slabs (down to one,
+                // 24 bytes per ray) where the table or the memory left is too small. (Samples past
+                // the last line are at most one.)
+                for (int cpd = tile;; cpd *= 2) {
+                    const bool deepest = !fast_ || cpd > maxDim;
+                    if (!deepest && !fits(cpd))
+                        continue;
+                    try {
+                        buildCheckpoints(cpd);
+                        break;
+                    } catch (const Error&) {
+                        if (deepest)
+                            throw;
+                        cudaGetLastError();
+                    }
+                }
             }
 
             // Per view and driving axis g: set bit 4+g of the view's axis word when neighbouring

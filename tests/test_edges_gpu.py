@@ -548,3 +548,30 @@ def test_siddon_copies_leave_the_adjoint_its_tables(cuda):
         proj.close()
         torch.cuda.empty_cache()
     assert np.array_equal(*out)
+
+
+def test_fast_joseph_2d_with_little_room_for_checkpoints(cuda, oracle):
+    """The forward of the `fast` operator, whose adjoint has no use for the checkpoint table, then
+    takes deeper slabs."""
+    import elsa_b200
+    torch = cuda
+    vol = (1000, 980)
+    poses, det, x, _ = _problem(oracle, vol, 1000, [1400])
+    make = lambda: elsa_b200.Projector(elsa_b200.PROJECTOR_JOSEPH, vol, det, poses, (1.0,))
+    proj = make()
+    ref = _apply(torch, proj, x, False)
+    proj.close()
+    d = torch.from_numpy(x).cuda()
+    y = torch.full((ref.size,), float("nan"), device="cuda")
+    # 45 MB of rays, 202 MB of checkpoints (one slab: 34 MB)
+    full = _fill_memory(torch, 160 << 20)
+    try:
+        proj = make()
+        proj.apply_ptr(d.data_ptr(), y.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    got = y.cpu().numpy()
+    assert rel_l2(got, ref) <= PARITY
+    assert not np.array_equal(got, ref)  # (the slabs' sums were added in another order)
