@@ -114,12 +114,15 @@ namespace elsa_b200
                      : "memory");
     }
 
-    // Correctly rounded quotients and square roots of pairs, by the residual-correction theorems of
-    // P. W. Markstein (IBM J. Res. Dev. 34(1), 1990): with y within half an ulp (and a little) of
-    // 1 / b and q within an ulp of a / b, q + (a - b q) y, rounded once, is a / b rounded;
-    // likewise for the root. They hold where no intermediate over- or underflows: for operands in
-    // midRange (a also 0). Compared with __fdiv_rn and __fsqrt_rn on 10^10 random operands per
-    // range (exponents within 2, 12 and 39 of 0): no difference.
+    // Correctly rounded quotients and square roots, by the residual corrections of P. W. Markstein
+    // (IBM J. Res. Dev. 34(1), 1990): with y = 1 / b rounded and q = a y rounded, q + (a - b q) y,
+    // rounded once, is a / b rounded; likewise for the root. They hold where no intermediate over-
+    // or underflows: for operands in midRange (a also 0). That one refinement of the approximate
+    // reciprocal gives the rounded one, and the whole sequence the rounded root, was compared for
+    // every float of the range, the quotient next to the rounding midpoints of every odd
+    // denominator, where it could go wrong (tests/test_rounding_gpu.py). A reciprocal refined from
+    // twice the half-reciprocal that the root leaves is not always the rounded one: a / sqrt(n2) then
+    // missed 30 of the 5e8 hardest quotients.
     __device__ __forceinline__ bool midRange(float a) // 2^-40 <= |a| <= 2^40
     {
         return fabsf(a) >= 9.0949470e-13f && fabsf(a) <= 1.0995116e12f;
@@ -139,17 +142,22 @@ namespace elsa_b200
         const float q = __fmul_rn(a, y);
         return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
     }
-    __device__ __forceinline__ float root(float a, float& h)
+    __device__ __forceinline__ float root(float a)
     {
         const float w = rsqrtf(a);
-        float g = __fmul_rn(a, w);
-        h = __fmul_rn(w, 0.5f);
+        float g = __fmul_rn(a, w), h = __fmul_rn(w, 0.5f);
         const float t = __fmaf_rn(-h, g, 0.5f);
         g = __fmaf_rn(g, t, g);
         h = __fmaf_rn(h, t, h);
         return __fmaf_rn(__fmaf_rn(-g, g, a), h, g);
     }
-    // 1 / b to half an ulp (and a little) from an approximation y.
+    // a / sqrt(n2), rounded twice; norm: sqrt(n2).
+    __device__ __forceinline__ float overRoot(float a, float n2, float& norm)
+    {
+        norm = root(n2);
+        return quotient(a, norm, refineRcp(norm, rcpApprox(norm)));
+    }
+    // 1 / b rounded, from an approximation y.
     __device__ __forceinline__ float2 refineRcp2(float2 b, float2 y)
     {
         return fma2(y, fma2(neg2(b), y, splat2(1.0f)), y);
@@ -160,12 +168,11 @@ namespace elsa_b200
         const float2 q = mul2(a, y);
         return fma2(fma2(neg2(b), q, a), y, q);
     }
-    // sqrt(a) rounded; h: half of its reciprocal, approximately.
-    __device__ __forceinline__ float2 root2(float2 a, float2& h)
+    // sqrt(a) rounded.
+    __device__ __forceinline__ float2 root2(float2 a)
     {
         const float2 w = make_float2(rsqrtf(a.x), rsqrtf(a.y));
-        float2 g = mul2(a, w);
-        h = mul2(w, splat2(0.5f));
+        float2 g = mul2(a, w), h = mul2(w, splat2(0.5f));
         const float2 t = fma2(neg2(h), g, splat2(0.5f));
         g = fma2(g, t, g);
         h = fma2(h, t, h);

@@ -452,10 +452,10 @@ namespace elsa_b200
                             const float2 v = sub2(diff[k], fma2(dot, splat2(rd[k]), zero));
                             sq = k == 0 ? fma2(v, v, zero) : add2(sq, fma2(v, v, zero));
                         }
-                        float2 dist, h;
+                        float2 dist;
                         // (a squared distance is below 2^40: volume edges are below 2^19)
                         if (fminf(sq.x, sq.y) >= 9.0949470e-13f)
-                            dist = root2(sq, h);
+                            dist = root2(sq);
                         else
                             dist = make_float2(sqrtf(sq.x), sqrtf(sq.y));
                         f(word, i + 1 < to[I],
