@@ -133,8 +133,8 @@ def _voxel_reference(oracle, kind, params, dim):
 @pytest.mark.parametrize("vol,views,det", [((13, 21, 9), 7, [17, 12]), ((50, 6, 49), 5, [70, 31]),
                                            ((200, 7), 6, [90]), ((60, 41), 11, [70])])
 def test_voxel_footprints(cuda, oracle, vol, views, det, kind, params, mode):
-    """Footprints of one pixel to more than six columns, lattices that overlap (shared atomics),
-    patches that do not fit, tables that do not end in 0, voxels projected off the detector. The
+    """Footprints of one pixel to more than six columns, detector patches that do not fit, tables
+    that do not end in 0, voxels projected off the detector (the small problems' forward). The
     default adjoint visits exactly the pixels of the exact one: its weights differ by a few ulp
     (an edge pixel more or less would show as 1e-4)."""
     import elsa_b200
@@ -575,3 +575,38 @@ def test_fast_joseph_2d_with_little_room_for_checkpoints(cuda, oracle):
     got = y.cpu().numpy()
     assert rel_l2(got, ref) <= PARITY
     assert not np.array_equal(got, ref)  # (the slabs' sums were added in another order)
+
+
+@pytest.mark.parametrize("kind", ["SIDDON", "BINARY"])
+@pytest.mark.parametrize("gamma", [0.0, 0.5 * np.pi])  # rays along z and along x
+def test_siddon_forward_beyond_32_bit_offsets(cuda, oracle, kind, gamma):
+    """A volume of 2^32 words and more, rays through its last planes: the same visits and sums, bit
+    for bit. (The host copy is zero pages but for a few planes.)"""
+    import elsa_b200
+    torch = cuda
+    vol, det = (1700, 1600, 1600), [12, 9, 1]
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB of device memory")
+    one = [1.0] * 3
+    pose = elsa_b200.pose_3d(9000.0, 2000.0, one, [850.5, 800.25, 1594.0], one, [6.0, 4.5, 0.0],
+                             gamma)
+    planes = [0, 1, 900, 1590, 1591, 1592, 1593, 1594, 1595, 1596, 1597, 1598, 1599]
+    size = vol[0] * vol[1]
+    assert size * vol[2] > 2 ** 32 > size * planes[2]
+    x = np.zeros(size * vol[2], np.float32)
+    d = torch.zeros(x.size, device="cuda")
+    rng = np.random.default_rng(8)
+    for k in planes:
+        part = rng.uniform(0.5, 1, size).astype(np.float32)
+        x[k * size:(k + 1) * size] = part
+        d[k * size:(k + 1) * size] = torch.from_numpy(part).cuda()
+    proj = elsa_b200.Projector(getattr(elsa_b200, "PROJECTOR_" + kind), vol, det, pose)
+    y = torch.full((proj.range_size,), float("nan"), device="cuda")
+    proj.apply_ptr(d.data_ptr(), y.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    fn = oracle.siddon if kind == "SIDDON" else oracle.binary
+    ref = np.asarray(fn(x, vol, det, pose), np.float32)
+    assert np.count_nonzero(ref) > ref.size // 2  # (rays along x at the volume's end may miss it)
+    assert np.array_equal(y.cpu().numpy(), ref)
+    del d
+    torch.cuda.empty_cache()
