@@ -394,7 +394,7 @@ def run_elsa(args):
     samples = proj.info(2)
     bytes_per_pass = 4.0 * (proj.domain_size + proj.range_size) + 16.0 * samples
     fwd_avg, adj_avg = fwd_ms / max(timed, 1), adj_ms / max(timed, 1)
-    dominant = "josephAdjointKernel" if adj_avg >= fwd_avg else "josephForwardKernel"
+    dominant = "josephAdjointAxisKernel" if adj_avg >= fwd_avg else "forwardTmaKernel"
     dom_ms = max(fwd_avg, adj_avg)
     peak, peak_kind = _peaks()
     achieved = bytes_per_pass / (dom_ms / 1e3) / 1e9

@@ -29,7 +29,7 @@
 // and weights of the forward kernel.
 // The launch knob kKnobAdjointScatter = 1 selects a thread-per-ray scatter instead (the forward's
 // sample loop with atomic adds to the four taps), slower in 2D (512^2 / 720 views: 1.74 ms against
-// 0.51) and 3D, where four global atomics per sample exceed what the L2 sustains. A shared-memory
+// 0.54) and 3D, where four global atomics per sample exceed what the L2 sustains. A shared-memory
 // variant (several warps per brick adding with shared atomics, no ray classes) measured 65.5 ms
 // against 54.8 ms at 256^3 / 360 views and was dropped.
 #include "joseph_tma.cuh"
@@ -587,7 +587,7 @@ namespace elsa_b200
         // exact accumulated positions of the checkpoints; the slabs' sums are added in slab
         // order. Bound by issue and L2 latency: one thread per ray reading the image itself took
         // 0.87 ms at 512^2 / 720 views / 730 pixels (half of the views read one word per sector),
-        // this takes 0.23 ms.
+        // this takes 0.24 ms.
         constexpr int kLinePad = 8;
         __host__ __device__ inline int linePitch(int n) { return (n + 2 * kLinePad + 3) / 4 * 4; }
 
@@ -731,7 +731,7 @@ namespace elsa_b200
         // are not written out). The NW warps of a block take views NW apart of the block's chunk;
         // their tiles are added in warp order, the chunks' partial images in chunk order.
         // Bound by the latency of the read-add-write chain of a step at 12 warps per SM (issue at
-        // 58 %, 28 instructions per step of 32 rays). 512^2 / 720 views / 730 pixels: 0.51 ms;
+        // 58 %, 28 instructions per step of 32 rays). 512^2 / 720 views / 730 pixels: 0.54 ms;
         // eight warps sharing a tile, merging taps by shuffles and adding in phases, took 1.99.
         template <int TILE>
         struct Tile2d {
@@ -937,9 +937,9 @@ namespace elsa_b200
         // of the brick grown by about half a voxel, holds few rays that miss it. One warp owns a
         // brick in shared memory for a chunk of views and splats the window's rays class by class:
         // rays of one class are more than two voxels apart, so no two lanes add to one word at
-        // once and the brick needs no atomics. A tap outside the brick is predicated off (the
-        // neighbouring brick owns it); with ELSA_AXIS_HALO 2 the brick instead carries a two-voxel
-        // halo into which tap indices are clamped, and the halo is not written out.
+        // once and the brick needs no atomics. Taps outside the brick belong to the neighbouring
+        // brick: those of rows are predicated off, those of columns fall into a halo column that
+        // is not written out.
         // ---------------------------------------------------------------------------------------
         // Shared-memory brick of TD planes (along G) of TV rows x TW columns. Columns run along
         // the non-driving axis over which the rays of a detector row spread (the warp's lanes
@@ -1248,8 +1248,8 @@ namespace elsa_b200
         // blocks; their rays start and end in more tiles).
         using Adjoint2dLarge = Adjoint2dConfig<64, 4>;
         using Adjoint2dSmall = Adjoint2dConfig<32, 8>;
-        // pixels up to which the tiles are the small ones (for 512^2 they are as fast, 0.504 ms against
-        // 0.514, but need twice the checkpoints)
+        // pixels up to which the tiles are the small ones: a larger image fills the GPU with the large
+        // ones, which need half the checkpoints (at 512^2 either takes the same, 0.504 ms and 0.514)
         constexpr int kSmallImage = 256 * 256;
         // Pixels, and pixels times views, up to which the forward reads the image itself. Padded /
         // direct in us, 1.45 pixels per column: 32^2 / 40 views 14.3 / 8.6; 80^2 / 180 (1.15e6)
@@ -1928,7 +1928,7 @@ namespace elsa_b200
             cudaTextureObject_t fastTex_ = 0;
             std::unique_ptr<DeviceBuffer> fastTable_;
             int scatter_ = 0; // 1: atomic scatter adjoint (2D: 512^2 / 720 views 1.74 ms
-                              // against 0.51; 3D 256^3 / 360 views 92 ms against 28.2)
+                              // against 0.54; 3D 256^3 / 360 views 92 ms against 28.2)
             JosephRay* dRays_ = nullptr;
             unsigned* dViewAxes_ = nullptr;
             RayWindow* dWindows_ = nullptr;

@@ -49,7 +49,7 @@ namespace elsa_b200
         double* partials;
     };
 
-    // The CGNE update (dot <c, q> -> den, step, norm, direction) of `count` instances in five
+    // The CGNE update (dot <c, q> -> den, step, norm, direction) of `count` instances in three
     // launches; every instance runs the blocks and summation order of the single-instance
     // launches (launchCgDen, launchCgStep, launchCgDirection), so its results
     // are bit-identical to theirs. entries: device array; maxN: largest n.
