@@ -181,6 +181,32 @@ def test_voxel_lattice(cuda, oracle, vol, views, det, kind, params, mode):
         assert rel_l2(_apply(cuda, proj, x, False), ref) <= PARITY
 
 
+@pytest.mark.parametrize("kind,params", VOXEL_KINDS)
+@pytest.mark.parametrize("offset", [(0.0, 0.0), (40.0, 0.0), (-25.0, 70.0), (400.0, 0.0)])
+@pytest.mark.parametrize("s2c,c2d", [(400.0, 100.0), (55.0, 40.0), (-300.0, 800.0), (20.0, 60.0)])
+@pytest.mark.parametrize("vol,views,det", [((50, 60, 49), 35, [24, 17]), ((200, 150), 16, [70])])
+def test_voxel_lattice_on_a_small_detector(cuda, oracle, vol, views, det, s2c, c2d, offset, kind,
+                                           params):
+    """Detectors that see a part of the volume or none of it: the ends of the lattice that project
+    off them are left out, from near and far sources, behind them and around them."""
+    import elsa_b200
+    one, origin, sino = [1.0] * len(vol), [0.5 * v for v in vol], [0.5 * d for d in det] + [0.0]
+    angles = np.linspace(0.0, 6.0, views)
+    if len(vol) == 3:
+        poses = [elsa_b200.pose_3d(s2c, c2d, one, origin, one, sino, g, pp_offset=offset)
+                 for g in angles]
+    else:
+        poses = [elsa_b200.pose_2d(s2c, c2d, g, one, origin, one, sino, pp_offset=offset[0])
+                 for g in angles]
+    poses, det = np.concatenate(poses), det + [views]
+    x = np.random.default_rng(6).uniform(0, 1, int(np.prod(vol))).astype(np.float32)
+    proj = elsa_b200.Projector(VOXEL_CODES[kind], vol, det, poses,
+                               tuple(map(float, params)) + (0,))
+    ref = oracle.voxel_project(False, x, vol, det, poses,
+                               *_voxel_reference(oracle, kind, params, len(vol)), 0)
+    assert rel_l2(_apply(cuda, proj, x, False), ref) <= PARITY
+
+
 @pytest.mark.parametrize("radius", [6.0, 9.0])
 @pytest.mark.parametrize("vol,views,det", LATTICE)
 def test_voxel_lattice_of_wide_footprints(cuda, oracle, vol, views, det, radius):
