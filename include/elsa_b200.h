@@ -165,7 +165,8 @@ elsa_status elsa_projector_destroy(elsa_projector* projector);
 elsa_status elsa_projector_sizes(const elsa_projector* projector, int64_t* domain_size,
                                  int64_t* range_size);
 
-/* Diagnostics: key 0 = conflict-free ray class spacing of the adjoint, 1 = adjoint bricks,
+/* Diagnostics: key 0 = conflict-free ray class spacing of the adjoint, 1 = adjoint bricks (voxel
+ * projectors: bricks of the small problems' forward),
  * 2 = samples per forward pass (sum over rays of the Joseph step count), 3 = error word of the
  * device pipeline (0 = no timed-out wait; synchronizes), 4 = detector tiles on the gather
  * fallback of the staged forward, in parts per million, 5 = footprint mode of a voxel

@@ -131,7 +131,8 @@ def _voxel_reference(oracle, kind, params, dim):
     ("blob", (9.0, 10.83, 2)), ("blob", (1.3, 2.0, 0)), ("bspline", (0,)), ("bspline", (5,)),
     ("phase_blob", (3.1, 10.83, 2)), ("phase_bspline", (3,))])
 @pytest.mark.parametrize("vol,views,det", [((13, 21, 9), 7, [17, 12]), ((50, 6, 49), 5, [70, 31]),
-                                           ((200, 7), 6, [90]), ((60, 41), 11, [70])])
+                                           ((200, 7), 6, [90]), ((60, 41), 11, [70]),
+                                           ((700, 500), 3, [900])])
 def test_voxel_footprints(cuda, oracle, vol, views, det, kind, params, mode):
     """Footprints of one pixel to more than six columns, detector patches that do not fit, tables
     that do not end in 0, voxels projected off the detector (the small problems' forward). The
@@ -184,7 +185,7 @@ def test_voxel_lattice(cuda, oracle, vol, views, det, kind, params, mode):
 @pytest.mark.parametrize("kind,params", VOXEL_KINDS)
 @pytest.mark.parametrize("offset", [(0.0, 0.0), (40.0, 0.0), (-25.0, 70.0), (400.0, 0.0)])
 @pytest.mark.parametrize("s2c,c2d", [(400.0, 100.0), (55.0, 40.0), (-300.0, 800.0), (20.0, 60.0)])
-@pytest.mark.parametrize("vol,views,det", [((50, 60, 49), 35, [24, 17]), ((200, 150), 16, [70])])
+@pytest.mark.parametrize("vol,views,det", [((50, 60, 49), 41, [24, 17]), ((200, 150), 16, [70])])
 def test_voxel_lattice_on_a_small_detector(cuda, oracle, vol, views, det, s2c, c2d, offset, kind,
                                            params):
     """Detectors that see a part of the volume or none of it: the ends of the lattice that project
